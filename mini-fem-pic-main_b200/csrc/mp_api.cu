@@ -320,6 +320,7 @@ int mp_destroy(mp_ctx *ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     adjoint_free(ctx);
     solve_free(ctx);
+    nd_free(ctx);
     output_free(ctx);  // joins a writer still running
     inject_free(ctx);
     sparse_free(ctx);
@@ -652,8 +653,10 @@ int mp_fe_setup(mp_ctx *ctx, const mp_fe_desc *fe) {
                    ctx->eq_a};
     for (void *p : old)
         if (p) cudaFree(p);
+    nd_free(ctx);
     ctx->J32 = ctx->K32 = nullptr;
     ctx->k32_current = false;
+    ctx->k_given = fe->K_rows || fe->K_dense;
     const long long ld = (neq + 31) & ~31ll;
     size_t vec = sizeof(double) * (size_t)(ld + 64);
     MP_CUDA(ctx, cudaMalloc(&ctx->ID, sizeof(int) * nn));
@@ -671,7 +674,7 @@ int mp_fe_setup(mp_ctx *ctx, const mp_fe_desc *fe) {
         MP_CUDA(ctx, cudaMemset(*p, 0, vec));
     }
     ctx->K = ctx->J = nullptr;  // J: allocated when an FP64 dense J is first built
-    ctx->j32_current = ctx->j_current = false;
+    ctx->j32_current = ctx->j_current = ctx->j_dense = ctx->fp_is_j = false;
     const bool dense = ctx->fe_storage == MP_FE_STORAGE_DENSE;
     if (dense) MP_CUDA(ctx, cudaMalloc(&ctx->K, sizeof(double) * (size_t)ld * neq));
     cudaStream_t st = ctx->stream;
@@ -748,6 +751,10 @@ int mp_fe_download(mp_ctx *ctx, int which, double *out) {
     if (which == MP_MAT_K || which == MP_MAT_J) {
         if (!ctx->fe_ready) return fail(ctx, MP_ERR_STATE, "no FE setup");
         if (!ctx->K) return fail(ctx, MP_ERR_STATE, "sparse storage: no dense matrix (mp_fe_sparse_matrix)");
+        if (which == MP_MAT_J && !ctx->j_dense && ctx->fp_is_j) {
+            int rc = fe_dense_j(ctx);
+            if (rc) return rc;
+        }
         if (which == MP_MAT_J && !ctx->J) return fail(ctx, MP_ERR_STATE, "no FP64 J built yet (mp_fe_build_j)");
         const long long ld = (ctx->neq + 31) & ~31ll;
         MP_CUDA(ctx, cudaMemcpy2DAsync(out, sizeof(double) * ctx->neq, which == MP_MAT_K ? ctx->K : ctx->J,
@@ -879,6 +886,12 @@ int mp_compute_phi(mp_ctx *ctx, const double *ion_den, int method, int form, mp_
     int rc;
     const double *den = den_source(ctx, ion_den, &rc);
     if (rc) return rc;
+    // the sparse direct solver needs neither the dense J nor its FP32 copy
+    bool nd = false;
+    const bool direct = method == MP_METHOD_LAPACK || (method == MP_METHOD_NONLINEAR && form == MP_FORM_MIXED);
+    if (direct && (form == MP_FORM_FP64 || ctx->mixed_factor == MP_MIXED_AUTO) &&
+        (rc = nd_prepare(ctx, form == MP_FORM_MIXED, &nd)))
+        return rc;
     cudaEventRecord(ctx->t0.a, ctx->stream);
     // solve(): y starts at zero and is reused across Newton iterations
     MP_CUDA(ctx, cudaMemsetAsync(ctx->y, 0, sizeof(double) * ctx->neq, ctx->stream));
@@ -894,7 +907,7 @@ int mp_compute_phi(mp_ctx *ctx, const double *ion_den, int method, int form, mp_
         for (it = 0; it < 10; it++) {
             if ((rc = fe_build_f1(ctx, den))) return rc;
             if ((rc = fe_residual(ctx))) return rc;
-            if ((rc = fe_build_j(ctx, method, form))) return rc;
+            if ((rc = fe_build_j(ctx, method, form, !nd))) return rc;
             rc = sparse                    ? fe_solve_cg(ctx, st)
                  : form == MP_FORM_FP64 ? fe_solve_gs(ctx, st)
                                         : fe_solve_ldlt(ctx, form, st);
@@ -917,7 +930,7 @@ int mp_compute_phi(mp_ctx *ctx, const double *ion_den, int method, int form, mp_
         // one Newton step, src/FESolver.cpp:301-317
         if ((rc = fe_build_f1(ctx, den))) return rc;
         if ((rc = fe_residual(ctx))) return rc;
-        if ((rc = fe_build_j(ctx, method, method == MP_METHOD_GAUSS_SEIDEL ? MP_FORM_FP64 : form))) return rc;
+        if ((rc = fe_build_j(ctx, method, method == MP_METHOD_GAUSS_SEIDEL ? MP_FORM_FP64 : form, !nd))) return rc;
         rc = method == MP_METHOD_SPARSE_CG      ? fe_solve_cg(ctx, st)
              : method == MP_METHOD_GAUSS_SEIDEL ? fe_solve_gs(ctx, st)
                                                 : fe_solve_ldlt(ctx, form, st);

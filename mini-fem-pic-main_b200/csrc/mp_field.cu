@@ -188,29 +188,52 @@ int fe_j32_from_k(mp_ctx *ctx) {
     return MP_OK;
 }
 
-int fe_build_j(mp_ctx *ctx, int method, int form) {
+// The dense FP64 J = K - diag(FP) from the current FP.
+int fe_dense_j(mp_ctx *ctx) {
+    const long long ld = (ctx->neq + 31) & ~31ll;
+    // neq^2 doubles, allocated on their first use
+    if (!ctx->J) MP_CUDA(ctx, cudaMalloc(&ctx->J, sizeof(double) * (size_t)ld * ctx->neq));
+    k_copy_j<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(ctx->neq, ld, ctx->K, ctx->FP, ctx->J), ++ctx->launches;
+    MP_CUDA(ctx, cudaGetLastError());
+    ctx->j_dense = true;
+    return MP_OK;
+}
+
+// as_array = false: the solver at hand takes J = K - diag(FP) from the sparse K
+// and FP, and the dense array is formed only if something asks for it.
+int fe_build_j(mp_ctx *ctx, int method, int form, bool as_array) {
     // the full symmetric J serves both dense solvers (Lapack reads only one
     // triangle); the sparse methods apply J = K - diag(FP) from K and FP
+    const bool fp64_j = ctx->K && method <= MP_METHOD_LAPACK && form == MP_FORM_FP64;
+    if (!fp64_j && ctx->j_current && !ctx->j_dense) {
+        // FP is about to change under an FP64 J that a later solve may still use
+        int rc = fe_dense_j(ctx);
+        if (rc) return rc;
+    }
     int th = 256;
     k_node_terms<<<(ctx->n_nodes + th - 1) / th, th, 0, ctx->stream>>>(
         ctx->n_nodes, ctx->ID, nullptr, ctx->d, 0.0, -QE / EPS0, ctx->n0, ctx->phi0, ctx->kTe, 1 / ctx->kTe,
         nullptr, ctx->work), ++ctx->launches;
     k_eq_gather<<<(ctx->neq + th - 1) / th, th, 0, ctx->stream>>>(ctx->neq, ctx->eq_ptr, ctx->eq_tet, ctx->eq_a,
                                                                  ctx->detJ, ctx->work, ctx->FP, 0), ++ctx->launches;
-    long long ld = (ctx->neq + 31) & ~31ll;
     if (method == MP_METHOD_SPARSE_CG || method == MP_METHOD_SPARSE_NEWTON || !ctx->K) {
         ctx->j32_current = false;
+        ctx->fp_is_j = false;
     } else if (form == MP_FORM_MIXED) {
         // the mixed form factors an FP32 copy and refines against K and FP: no FP64 J
-        int rc = fe_j32_from_k(ctx);
-        if (rc) return rc;
-        ctx->j32_current = true;
-    } else {
-        // the FP64 J (neq^2 doubles) is allocated on its first use
-        if (!ctx->J) MP_CUDA(ctx, cudaMalloc(&ctx->J, sizeof(double) * (size_t)ld * ctx->neq));
-        k_copy_j<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(ctx->neq, ld, ctx->K, ctx->FP, ctx->J), ++ctx->launches;
+        ctx->fp_is_j = false;
         ctx->j32_current = false;
+        if (as_array) {
+            int rc = fe_j32_from_k(ctx);
+            if (rc) return rc;
+            ctx->j32_current = true;
+        }
+    } else {
+        ctx->j32_current = false;
+        ctx->j_dense = false;
         ctx->j_current = true;
+        ctx->fp_is_j = true;
+        if (as_array) return fe_dense_j(ctx);
     }
     MP_CUDA(ctx, cudaGetLastError());
     return MP_OK;

@@ -172,7 +172,15 @@ struct mp_ctx {
     float *K32 = nullptr;                 // [neq][neq] K's lower triangle in FP32 (the mixed form's J32 source)
     bool k32_current = false;             // K32 holds the current K
     bool j32_current = false;             // J32 holds the lower triangle of the current J
-    bool j_current = false;               // J holds the current J (not yet overwritten by its factor)
+    bool j_current = false;               // an FP64 J has been built and not yet used up by a factorization
+    bool j_dense = false;                 // the array J holds it (else it is K - diag(FP), formed when needed)
+    bool fp_is_j = false;                 // FP is the current FP64 J's diagonal term
+    bool k_given = false;                 // K came from the caller, not from the mesh
+    void *nd = nullptr;                   // sparse direct solver (mp_nd.cu)
+    // K's pattern on the host until the sparse direct solver's plan is made
+    // (dense storage): CSR rows, columns ascending, and each entry's slot in sp_val
+    std::vector<long long> csr_ptr, csr_slot;
+    std::vector<int> csr_col;
     double *scal = nullptr;               // device scalars for reductions
     double *scal_host = nullptr;          // pinned
     int *eq_ptr = nullptr, *eq_tet = nullptr;   // CSR equation -> (tet, a) sorted by tet
@@ -247,7 +255,12 @@ int launch_update_ef(mp_ctx *ctx);
 
 int fe_build_f1(mp_ctx *ctx, const double *den_dev);
 int fe_residual(mp_ctx *ctx);
-int fe_build_j(mp_ctx *ctx, int method, int form = MP_FORM_FP64);
+int fe_build_j(mp_ctx *ctx, int method, int form = MP_FORM_FP64, bool as_array = true);
+int fe_dense_j(mp_ctx *ctx);
+int nd_prepare(mp_ctx *ctx, bool mixed, bool *usable);
+int nd_factor_solve(mp_ctx *ctx, const double *b, double *y);
+int nd_solve_add(mp_ctx *ctx, const double *b, double *y);
+void nd_free(mp_ctx *ctx);
 int fe_j32_from_k(mp_ctx *ctx);
 int fe_solve_ldlt(mp_ctx *ctx, int form, mp_newton_stats *st);
 int fe_solve_gs(mp_ctx *ctx, mp_newton_stats *st);

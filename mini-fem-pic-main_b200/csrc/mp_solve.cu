@@ -151,17 +151,66 @@ static int ensure_scratch(mp_ctx *ctx, SolveScratch **out) {
 // accuracy, so y matches dsysv_'s to the FP64 form's tolerance.
 constexpr double REFINE_RTOL = 1e-14;
 
+// A residual above this share of ||G|| (an indefinite J can meet a bad pivot
+// order) sends the sparse factorization's solve to the dense one.
+constexpr double SPARSE_RTOL = 1e-9;
+
+// The direct solve by the sparse factorization; *done is false when the dense
+// one has to take it over (a zero or non-finite pivot, a poor residual).
+static int solve_nd(mp_ctx *ctx, int form, mp_newton_stats *st, bool *done) {
+    *done = false;
+    cudaEventRecord(ctx->t1.a, ctx->stream);
+    int rc = nd_factor_solve(ctx, ctx->G, ctx->y);
+    if (rc) return rc;
+    cudaEventRecord(ctx->t1.b, ctx->stream);
+    double rn = 0, bn = 0, prev = 1e300;
+    int it = 1;
+    for (; it < 60; it++) {
+        if ((rc = resid_norms(ctx, ctx->y, ctx->G, ctx->work, nullptr, &rn, &bn))) return rc;
+        if (form == MP_FORM_FP64 || !(rn > REFINE_RTOL * bn) || !(rn <= SPARSE_RTOL * bn) || rn > 0.7 * prev) break;
+        prev = rn;
+        if ((rc = nd_solve_add(ctx, ctx->work, ctx->y))) return rc;
+    }
+    unsigned long long bad = 0;
+    if ((rc = check_flags(ctx, FLAG_SINGULAR | FLAG_LOOKBACK_TIMEOUT, &bad))) return rc;
+    if (bad & FLAG_LOOKBACK_TIMEOUT)
+        return fail(ctx, MP_ERR_TIMEOUT, "a bounded wait in the factorization or the triangular solves gave up");
+    if (bad || !(rn <= SPARSE_RTOL * bn)) return MP_OK;
+    if (st) {
+        st->linear_iterations = it;
+        st->linear_residual = rn / ctx->neq;
+        float ms = 0;
+        cudaEventElapsedTime(&ms, ctx->t1.a, ctx->t1.b);
+        st->ms_factor = ms;
+    }
+    *done = true;
+    return MP_OK;
+}
+
 int fe_solve_ldlt(mp_ctx *ctx, int form, mp_newton_stats *st) {
+    int rc;
+    if (form == MP_FORM_FP64 && !ctx->j_current) return fail(ctx, MP_ERR_STATE, "no current FP64 J (build it first)");
+    bool nd = false;
+    if ((form == MP_FORM_FP64 ? ctx->fp_is_j : ctx->mixed_factor == MP_MIXED_AUTO) &&
+        (rc = nd_prepare(ctx, form == MP_FORM_MIXED, &nd)))
+        return rc;
+    if (nd) {
+        if ((rc = solve_nd(ctx, form, st, &nd))) return rc;
+        if (nd) {
+            if (form == MP_FORM_FP64) ctx->j_current = false;  // one solve a build of J
+            return MP_OK;
+        }
+    }
     SolveScratch *sp = nullptr;
-    int rc = ensure_scratch(ctx, &sp);
+    rc = ensure_scratch(ctx, &sp);
     if (rc) return rc;
     SolveScratch &sc = *sp;
     const int n = ctx->neq;
     const long long ld = (n + 31) & ~31ll;
     cudaEventRecord(ctx->t1.a, ctx->stream);
     if (form == MP_FORM_FP64) {
-        if (!ctx->J || !ctx->j_current) return fail(ctx, MP_ERR_STATE, "no current FP64 J (build it first)");
-        ctx->j_current = false;  // the factorization overwrites J
+        if (!ctx->j_dense && (rc = fe_dense_j(ctx))) return rc;
+        ctx->j_current = ctx->j_dense = false;  // the factorization overwrites J
         MP_CUDA(ctx, cudaMemcpyAsync(ctx->y, ctx->G, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
         LdltWork<double> w{sc.dvec64, sc.W64, sc.s64, sc.kt64, sc.Linv64, sc.Mc64, sc.ll, nullptr};
         rc = ldlt_factor_solve<double>(ctx, ctx->J, ld, n, ctx->y, w, true);
@@ -552,10 +601,11 @@ __global__ void k_gs_resid(int neq, long long ld, const double *__restrict__ A, 
 }
 
 int fe_solve_gs(mp_ctx *ctx, mp_newton_stats *st) {
-    if (!ctx->J || !ctx->j_current) return fail(ctx, MP_ERR_STATE, "no current FP64 J (build it first)");
+    if (!ctx->j_current) return fail(ctx, MP_ERR_STATE, "no current FP64 J (build it first)");
     SolveScratch *sp = nullptr;
     int rc = ensure_scratch(ctx, &sp);
     if (rc) return rc;
+    if (!ctx->j_dense && (rc = fe_dense_j(ctx))) return rc;
     const int n = ctx->neq;
     const long long ld = (n + 31) & ~31ll;
     const int nblk = (n + NB - 1) / NB;

@@ -467,23 +467,25 @@ int sparse_setup(mp_ctx *ctx, const std::vector<int> &LM, const std::vector<int>
     sparse_free(ctx);
     const int neq = ctx->neq;
     const int slices = (neq + 31) / 32;
-    std::vector<int> len(neq), cols;
-    std::vector<std::vector<int>> rows(neq);
-    long long nnz = 0;
+    std::vector<int> len(neq), cols, seen(neq, -1);
+    std::vector<long long> rowp(neq + 1, 0);
+    cols.reserve(16 * (size_t)neq);
     for (int P = 0; P < neq; P++) {
-        std::vector<int> &c = rows[P];
-        c.reserve(4 * (eq_ptr[P + 1] - eq_ptr[P]));
-        c.push_back(P);
+        cols.push_back(P);
+        seen[P] = P;
         for (int k = eq_ptr[P]; k < eq_ptr[P + 1]; k++)
             for (int b = 0; b < 4; b++) {
                 int Q = LM[4 * (size_t)eq_tet[k] + b];
-                if (Q >= 0) c.push_back(Q);
+                if (Q >= 0 && seen[Q] != P) {
+                    seen[Q] = P;
+                    cols.push_back(Q);
+                }
             }
-        std::sort(c.begin(), c.end());
-        c.erase(std::unique(c.begin(), c.end()), c.end());
-        len[P] = (int)c.size();
-        nnz += len[P];
+        std::sort(cols.begin() + rowp[P], cols.end());
+        rowp[P + 1] = (long long)cols.size();
+        len[P] = (int)(rowp[P + 1] - rowp[P]);
     }
+    const long long nnz = rowp[neq];
     std::vector<long long> ptr(slices + 1, 0);
     for (int s = 0; s < slices; s++) {
         int w = 0;
@@ -497,7 +499,7 @@ int sparse_setup(mp_ctx *ctx, const std::vector<int> &LM, const std::vector<int>
         for (int l = 0; l < 32; l++) {
             const int P = 32 * s + l;
             for (int k = 0; k < w; k++)
-                col[ptr[s] + 32ll * k + l] = P < neq ? (k < len[P] ? rows[P][k] : P) : 0;
+                col[ptr[s] + 32ll * k + l] = P < neq ? (k < len[P] ? cols[rowp[P] + k] : P) : 0;
         }
     }
     MP_CUDA(ctx, cudaMalloc(&ctx->sp_len, sizeof(int) * std::max(1, neq)));
@@ -510,6 +512,17 @@ int sparse_setup(mp_ctx *ctx, const std::vector<int> &LM, const std::vector<int>
     MP_CUDA(ctx, cudaMemset(ctx->sp_val, 0, sizeof(double) * std::max(1ll, slots)));
     ctx->sp_nnz = nnz;
     ctx->sp_slots = slots;
+    ctx->csr_ptr.clear();
+    ctx->csr_col.clear();
+    ctx->csr_slot.clear();
+    if (ctx->fe_storage == MP_FE_STORAGE_DENSE) {
+        ctx->csr_slot.resize(nnz);
+        for (int P = 0; P < neq; P++)
+            for (long long k = rowp[P]; k < rowp[P + 1]; k++)
+                ctx->csr_slot[k] = ptr[P >> 5] + 32ll * (k - rowp[P]) + (P & 31);
+        ctx->csr_ptr = std::move(rowp);
+        ctx->csr_col = std::move(cols);
+    }
     return MP_OK;
 }
 
