@@ -321,6 +321,7 @@ int mp_destroy(mp_ctx *ctx) {
     adjoint_free(ctx);
     solve_free(ctx);
     nd_free(ctx);
+    gs_free(ctx);
     output_free(ctx);  // joins a writer still running
     inject_free(ctx);
     sparse_free(ctx);
@@ -654,6 +655,8 @@ int mp_fe_setup(mp_ctx *ctx, const mp_fe_desc *fe) {
     for (void *p : old)
         if (p) cudaFree(p);
     nd_free(ctx);
+    gs_free(ctx);
+    ctx->k_fits = -1;
     ctx->J32 = ctx->K32 = nullptr;
     ctx->k32_current = false;
     ctx->k_given = fe->K_rows || fe->K_dense;
@@ -886,12 +889,13 @@ int mp_compute_phi(mp_ctx *ctx, const double *ion_den, int method, int form, mp_
     int rc;
     const double *den = den_source(ctx, ion_den, &rc);
     if (rc) return rc;
-    // the sparse direct solver needs neither the dense J nor its FP32 copy
-    bool nd = false;
-    const bool direct = method == MP_METHOD_LAPACK || (method == MP_METHOD_NONLINEAR && form == MP_FORM_MIXED);
-    if (direct && (form == MP_FORM_FP64 || ctx->mixed_factor == MP_MIXED_AUTO) &&
-        (rc = nd_prepare(ctx, form == MP_FORM_MIXED, &nd)))
-        return rc;
+    // the sparse solvers need neither the dense J nor its FP32 copy
+    bool lean = false;
+    const bool gs = method == MP_METHOD_GAUSS_SEIDEL || (method == MP_METHOD_NONLINEAR && form == MP_FORM_FP64);
+    if (gs) rc = gs_prepare(ctx, &lean);
+    else if (!sparse && (form == MP_FORM_FP64 || ctx->mixed_factor == MP_MIXED_AUTO))
+        rc = nd_prepare(ctx, form == MP_FORM_MIXED, &lean);
+    if (rc) return rc;
     cudaEventRecord(ctx->t0.a, ctx->stream);
     // solve(): y starts at zero and is reused across Newton iterations
     MP_CUDA(ctx, cudaMemsetAsync(ctx->y, 0, sizeof(double) * ctx->neq, ctx->stream));
@@ -907,7 +911,7 @@ int mp_compute_phi(mp_ctx *ctx, const double *ion_den, int method, int form, mp_
         for (it = 0; it < 10; it++) {
             if ((rc = fe_build_f1(ctx, den))) return rc;
             if ((rc = fe_residual(ctx))) return rc;
-            if ((rc = fe_build_j(ctx, method, form, !nd))) return rc;
+            if ((rc = fe_build_j(ctx, method, form, !lean))) return rc;
             rc = sparse                    ? fe_solve_cg(ctx, st)
                  : form == MP_FORM_FP64 ? fe_solve_gs(ctx, st)
                                         : fe_solve_ldlt(ctx, form, st);
@@ -930,7 +934,7 @@ int mp_compute_phi(mp_ctx *ctx, const double *ion_den, int method, int form, mp_
         // one Newton step, src/FESolver.cpp:301-317
         if ((rc = fe_build_f1(ctx, den))) return rc;
         if ((rc = fe_residual(ctx))) return rc;
-        if ((rc = fe_build_j(ctx, method, method == MP_METHOD_GAUSS_SEIDEL ? MP_FORM_FP64 : form, !nd))) return rc;
+        if ((rc = fe_build_j(ctx, method, method == MP_METHOD_GAUSS_SEIDEL ? MP_FORM_FP64 : form, !lean))) return rc;
         rc = method == MP_METHOD_SPARSE_CG      ? fe_solve_cg(ctx, st)
              : method == MP_METHOD_GAUSS_SEIDEL ? fe_solve_gs(ctx, st)
                                                 : fe_solve_ldlt(ctx, form, st);

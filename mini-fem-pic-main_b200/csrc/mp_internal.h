@@ -176,9 +176,10 @@ struct mp_ctx {
     bool j_dense = false;                 // the array J holds it (else it is K - diag(FP), formed when needed)
     bool fp_is_j = false;                 // FP is the current FP64 J's diagonal term
     bool k_given = false;                 // K came from the caller, not from the mesh
+    int k_fits = -1;                      // a given K is symmetric and of the mesh's pattern (-1: not looked at)
     void *nd = nullptr;                   // sparse direct solver (mp_nd.cu)
-    // K's pattern on the host until the sparse direct solver's plan is made
-    // (dense storage): CSR rows, columns ascending, and each entry's slot in sp_val
+    void *gs = nullptr;                   // sparse Gauss-Seidel solver (mp_gs.cu)
+    // K's pattern on the host, for the plans of the two (dense storage): CSR rows, columns ascending, and each entry's slot in sp_val
     std::vector<long long> csr_ptr, csr_slot;
     std::vector<int> csr_col;
     double *scal = nullptr;               // device scalars for reductions
@@ -261,6 +262,10 @@ int nd_prepare(mp_ctx *ctx, bool mixed, bool *usable);
 int nd_factor_solve(mp_ctx *ctx, const double *b, double *y);
 int nd_solve_add(mp_ctx *ctx, const double *b, double *y);
 void nd_free(mp_ctx *ctx);
+int gs_prepare(mp_ctx *ctx, bool *usable);
+int gs_solve(mp_ctx *ctx, double tol, mp_newton_stats *st);
+void gs_free(mp_ctx *ctx);
+int fe_pattern_fits(mp_ctx *ctx, bool *fits);
 int fe_j32_from_k(mp_ctx *ctx);
 int fe_solve_ldlt(mp_ctx *ctx, int form, mp_newton_stats *st);
 int fe_solve_gs(mp_ctx *ctx, mp_newton_stats *st);

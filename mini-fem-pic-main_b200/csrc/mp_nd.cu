@@ -940,33 +940,6 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
     }
 }
 
-// Whether a dense K (leading dimension ld) is symmetric and zero outside the
-// sparse pattern: counts[0] entries differing from their mirror image,
-// counts[1] the nonzeros.
-__global__ void k_nd_check_dense(int n, long long ld, const double *__restrict__ K, unsigned long long *counts) {
-    unsigned long long asym = 0, nz = 0;
-    const long long total = (long long)n * n;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const long long r = i / n, c = i - r * n;
-        const double v = K[r * ld + c];
-        if (v != 0.0) {
-            nz++;
-            if (!(v == K[c * ld + r])) asym++;
-        }
-    }
-    if (asym) atomicAdd(&counts[0], asym);
-    if (nz) atomicAdd(&counts[1], nz);
-}
-__global__ void k_nd_count_sparse(int neq, const int *__restrict__ len, const long long *__restrict__ ptr,
-                                  const double *__restrict__ val, unsigned long long *counts) {
-    const int P = blockIdx.x * blockDim.x + threadIdx.x;
-    if (P >= neq) return;
-    const long long base = ptr[P >> 5] + (P & 31);
-    unsigned long long nz = 0;
-    for (int k = 0; k < len[P]; k++) nz += val[base + 32ll * k] != 0.0;
-    atomicAdd(&counts[2], nz);
-}
-
 struct NdState {
     bool usable = false;               // the plan exists and is the faster way
     NdPlan plan;                       // (its host lists are dropped once on the device)
@@ -1019,21 +992,9 @@ int nd_prepare(mp_ctx *ctx, bool mixed, bool *usable) {
         s = new NdState();
         ctx->nd = s;
         const int n = ctx->neq;
-        const long long ld = (n + 31) & ~31ll;
-        bool fits = true;
-        if (ctx->k_given) {
-            unsigned long long *cnt = nullptr, h[3] = {0, 0, 0};
-            MP_CUDA(ctx, cudaMalloc(&cnt, sizeof(h)));
-            cudaMemsetAsync(cnt, 0, sizeof(h), ctx->stream);
-            k_nd_check_dense<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(n, ld, ctx->K, cnt), ++ctx->launches;
-            k_nd_count_sparse<<<(n + 255) / 256, 256, 0, ctx->stream>>>(n, ctx->sp_len, ctx->sp_ptr, ctx->sp_val, cnt),
-                ++ctx->launches;
-            cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
-            cudaError_t e = cudaStreamSynchronize(ctx->stream);
-            cudaFree(cnt);
-            MP_CUDA(ctx, e);
-            fits = h[0] == 0 && h[1] == h[2];
-        }
+        bool fits = false;
+        int rc = fe_pattern_fits(ctx, &fits);
+        if (rc) return rc;
         if (fits && !ctx->csr_ptr.empty()) {
             std::vector<double> pos(3 * (size_t)n, 0.0), npos(3 * (size_t)ctx->n_nodes);
             std::vector<int> ID(ctx->n_nodes);

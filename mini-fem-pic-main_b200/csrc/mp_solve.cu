@@ -602,14 +602,18 @@ __global__ void k_gs_resid(int neq, long long ld, const double *__restrict__ A, 
 
 int fe_solve_gs(mp_ctx *ctx, mp_newton_stats *st) {
     if (!ctx->j_current) return fail(ctx, MP_ERR_STATE, "no current FP64 J (build it first)");
+    const double tol = 1e-4;
+    int rc;
+    bool lean = false;
+    if (ctx->fp_is_j && (rc = gs_prepare(ctx, &lean))) return rc;
+    if (lean) return gs_solve(ctx, tol, st);
     SolveScratch *sp = nullptr;
-    int rc = ensure_scratch(ctx, &sp);
+    rc = ensure_scratch(ctx, &sp);
     if (rc) return rc;
     if (!ctx->j_dense && (rc = fe_dense_j(ctx))) return rc;
     const int n = ctx->neq;
     const long long ld = (n + 31) & ~31ll;
     const int nblk = (n + NB - 1) / NB;
-    const double tol = 1e-4;
     const int th = 256;
     const long long bl = ((long long)n * 32 + th - 1) / th;
     unsigned long long *flags = ctx->counters + C_FLAGS;

@@ -553,6 +553,56 @@ int fe_sparse_from_dense(mp_ctx *ctx) {
     return MP_OK;
 }
 
+// Whether a dense K (leading dimension ld) is symmetric and zero outside the
+// sparse pattern: counts[0] entries differing from their mirror image,
+// counts[1] the nonzeros.
+__global__ void k_check_dense(int n, long long ld, const double *__restrict__ K, unsigned long long *counts) {
+    unsigned long long asym = 0, nz = 0;
+    const long long total = (long long)n * n;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const long long r = i / n, c = i - r * n;
+        const double v = K[r * ld + c];
+        if (v != 0.0) {
+            nz++;
+            if (!(v == K[c * ld + r])) asym++;
+        }
+    }
+    if (asym) atomicAdd(&counts[0], asym);
+    if (nz) atomicAdd(&counts[1], nz);
+}
+__global__ void k_count_sparse(int neq, const int *__restrict__ len, const long long *__restrict__ ptr,
+                                  const double *__restrict__ val, unsigned long long *counts) {
+    const int P = blockIdx.x * blockDim.x + threadIdx.x;
+    if (P >= neq) return;
+    const long long base = ptr[P >> 5] + (P & 31);
+    unsigned long long nz = 0;
+    for (int k = 0; k < len[P]; k++) nz += val[base + 32ll * k] != 0.0;
+    atomicAdd(&counts[2], nz);
+}
+
+// Whether K is symmetric with no entry outside the mesh's pattern, so that a
+// solver may take J from the sparse K: a K assembled from the mesh is, one from
+// the caller is looked over (once).
+int fe_pattern_fits(mp_ctx *ctx, bool *fits) {
+    if (ctx->k_given && ctx->k_fits < 0) {
+        const int n = ctx->neq;
+        const long long ld = (n + 31) & ~31ll;
+        unsigned long long *cnt = nullptr, h[3] = {0, 0, 0};
+        MP_CUDA(ctx, cudaMalloc(&cnt, sizeof(h)));
+        cudaMemsetAsync(cnt, 0, sizeof(h), ctx->stream);
+        k_check_dense<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(n, ld, ctx->K, cnt), ++ctx->launches;
+        k_count_sparse<<<(n + 255) / 256, 256, 0, ctx->stream>>>(n, ctx->sp_len, ctx->sp_ptr, ctx->sp_val, cnt),
+            ++ctx->launches;
+        cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
+        cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        cudaFree(cnt);
+        MP_CUDA(ctx, e);
+        ctx->k_fits = h[0] == 0 && h[1] == h[2];
+    }
+    *fits = !ctx->k_given || ctx->k_fits > 0;
+    return MP_OK;
+}
+
 // K given on the host, sparse storage only: gather the nonzeros on the host.
 int fe_sparse_from_host(mp_ctx *ctx, const double *const *rows, const double *dense) {
     const int neq = ctx->neq;
