@@ -329,7 +329,7 @@ int mp_destroy(mp_ctx *ctx) {
                    ctx->den, ctx->den_fixed, ctx->counters, ctx->scal, ctx->compact_off, ctx->sort_hist,
                    ctx->part_block[0], ctx->part_block[1], ctx->ID, ctx->LM, ctx->detJ, ctx->nx, ctx->g, ctx->uh,
                    ctx->d, ctx->F0, ctx->F1, ctx->G, ctx->y, ctx->fvec, ctx->FP, ctx->work, ctx->K, ctx->J,
-                   ctx->J32, ctx->K32, ctx->eq_ptr, ctx->eq_tet, ctx->eq_a, ctx->gs_minv, ctx->den_in, ctx->dstage};
+                   ctx->J32, ctx->K32, ctx->eq_ptr, ctx->eq_tet, ctx->eq_a, ctx->eq_node, ctx->gs_minv, ctx->den_in, ctx->dstage};
     for (void *p : dev)
         if (p) cudaFree(p);
     if (ctx->counters_host) cudaFreeHost(ctx->counters_host);
@@ -648,10 +648,19 @@ int mp_fe_setup(mp_ctx *ctx, const mp_fe_desc *fe) {
             eq_tet[k] = e;
             eq_a[k] = (unsigned char)a;
         }
+    std::vector<int> eq_node(neq, -1);
+    ctx->one_node_each = true;
+    for (int n = 0; n < nn; n++)
+        if (fe->ID[n] >= 0) {
+            if (eq_node[fe->ID[n]] >= 0) ctx->one_node_each = false;
+            eq_node[fe->ID[n]] = n;
+        }
+    for (int A = 0; A < neq; A++)
+        if (eq_node[A] < 0) ctx->one_node_each = false;
     // (re)allocate
     void *old[] = {ctx->ID, ctx->LM, ctx->detJ, ctx->nx, ctx->g, ctx->uh, ctx->d, ctx->F0, ctx->F1, ctx->G, ctx->y,
                    ctx->fvec, ctx->FP, ctx->work, ctx->K, ctx->J, ctx->J32, ctx->K32, ctx->eq_ptr, ctx->eq_tet,
-                   ctx->eq_a};
+                   ctx->eq_a, ctx->eq_node};
     for (void *p : old)
         if (p) cudaFree(p);
     nd_free(ctx);
@@ -671,6 +680,7 @@ int mp_fe_setup(mp_ctx *ctx, const mp_fe_desc *fe) {
     MP_CUDA(ctx, cudaMalloc(&ctx->eq_ptr, sizeof(int) * (neq + 1)));
     MP_CUDA(ctx, cudaMalloc(&ctx->eq_tet, sizeof(int) * std::max(1, cnt[neq])));
     MP_CUDA(ctx, cudaMalloc(&ctx->eq_a, std::max(1, cnt[neq])));
+    MP_CUDA(ctx, cudaMalloc(&ctx->eq_node, sizeof(int) * neq));
     double **vp[] = {&ctx->d, &ctx->F0, &ctx->F1, &ctx->G, &ctx->y, &ctx->fvec, &ctx->FP, &ctx->work};
     for (double **p : vp) {
         MP_CUDA(ctx, cudaMalloc(p, vec));
@@ -687,6 +697,7 @@ int mp_fe_setup(mp_ctx *ctx, const mp_fe_desc *fe) {
     MP_CUDA(ctx, cudaMemcpyAsync(ctx->nx, fe->nx, sizeof(double) * 12 * nt, cudaMemcpyHostToDevice, st));
     MP_CUDA(ctx, cudaMemcpyAsync(ctx->g, fe->g, sizeof(double) * nn, cudaMemcpyHostToDevice, st));
     MP_CUDA(ctx, cudaMemcpyAsync(ctx->uh, fe->g, sizeof(double) * nn, cudaMemcpyHostToDevice, st));
+    MP_CUDA(ctx, cudaMemcpyAsync(ctx->eq_node, eq_node.data(), sizeof(int) * neq, cudaMemcpyHostToDevice, st));
     MP_CUDA(ctx, cudaMemcpyAsync(ctx->eq_ptr, cnt.data(), sizeof(int) * (neq + 1), cudaMemcpyHostToDevice, st));
     if (cnt[neq]) {
         MP_CUDA(ctx, cudaMemcpyAsync(ctx->eq_tet, eq_tet.data(), sizeof(int) * cnt[neq], cudaMemcpyHostToDevice, st));
@@ -895,10 +906,12 @@ int mp_compute_phi(mp_ctx *ctx, const double *ion_den, int method, int form, mp_
     if (gs) rc = gs_prepare(ctx, &lean);
     else if (!sparse && (form == MP_FORM_FP64 || ctx->mixed_factor == MP_MIXED_AUTO))
         rc = nd_prepare(ctx, form == MP_FORM_MIXED, &lean);
+    else lean = sparse;
     if (rc) return rc;
+    lean = lean && ctx->one_node_each;
     cudaEventRecord(ctx->t0.a, ctx->stream);
     // solve(): y starts at zero and is reused across Newton iterations
-    MP_CUDA(ctx, cudaMemsetAsync(ctx->y, 0, sizeof(double) * ctx->neq, ctx->stream));
+    if (!lean) MP_CUDA(ctx, cudaMemsetAsync(ctx->y, 0, sizeof(double) * ctx->neq, ctx->stream));
     double ms_factor = 0;
     if (method == MP_METHOD_NONLINEAR || method == MP_METHOD_SPARSE_NEWTON) {
         // solveNonLinear, src/FESolver.cpp:324-364: up to 10 Newton iterations,
@@ -909,15 +922,19 @@ int mp_compute_phi(mp_ctx *ctx, const double *ion_den, int method, int form, mp_
         double L2 = 0;
         int it;
         for (it = 0; it < 10; it++) {
-            if ((rc = fe_build_f1(ctx, den))) return rc;
-            if ((rc = fe_residual(ctx))) return rc;
-            if ((rc = fe_build_j(ctx, method, form, !lean))) return rc;
-            rc = sparse                    ? fe_solve_cg(ctx, st)
-                 : form == MP_FORM_FP64 ? fe_solve_gs(ctx, st)
-                                        : fe_solve_ldlt(ctx, form, st);
-            if (rc) return rc;
+            if (lean) {
+                if ((rc = fe_step_lean(ctx, den, method, form, it == 0, st, &L2))) return rc;
+            } else {
+                if ((rc = fe_build_f1(ctx, den))) return rc;
+                if ((rc = fe_residual(ctx))) return rc;
+                if ((rc = fe_build_j(ctx, method, form))) return rc;
+                rc = sparse                    ? fe_solve_cg(ctx, st)
+                     : form == MP_FORM_FP64 ? fe_solve_gs(ctx, st)
+                                            : fe_solve_ldlt(ctx, form, st);
+                if (rc) return rc;
+                if ((rc = fe_update_d(ctx, &L2))) return rc;
+            }
             ms_factor += st->ms_factor;
-            if ((rc = fe_update_d(ctx, &L2))) return rc;
             if (L2 < 1e-2) {
                 converged = true;
                 break;
@@ -925,26 +942,30 @@ int mp_compute_phi(mp_ctx *ctx, const double *ion_den, int method, int form, mp_
         }
         st->newton_iterations = converged ? it + 1 : it;
         st->l2 = L2;
-        if ((rc = fe_uh(ctx))) return rc;
+        if (!lean && (rc = fe_uh(ctx))) return rc;
         if (!converged) {
             MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             return fail(ctx, MP_ERR_NOT_CONVERGED, "NR failed to converge");
         }
     } else {
         // one Newton step, src/FESolver.cpp:301-317
-        if ((rc = fe_build_f1(ctx, den))) return rc;
-        if ((rc = fe_residual(ctx))) return rc;
-        if ((rc = fe_build_j(ctx, method, method == MP_METHOD_GAUSS_SEIDEL ? MP_FORM_FP64 : form, !lean))) return rc;
-        rc = method == MP_METHOD_SPARSE_CG      ? fe_solve_cg(ctx, st)
-             : method == MP_METHOD_GAUSS_SEIDEL ? fe_solve_gs(ctx, st)
-                                                : fe_solve_ldlt(ctx, form, st);
-        if (rc) return rc;
-        ms_factor = st->ms_factor;
         double L2 = 0;
-        if ((rc = fe_update_d(ctx, &L2))) return rc;
+        if (lean) {
+            if ((rc = fe_step_lean(ctx, den, method, form, true, st, &L2))) return rc;
+        } else {
+            if ((rc = fe_build_f1(ctx, den))) return rc;
+            if ((rc = fe_residual(ctx))) return rc;
+            if ((rc = fe_build_j(ctx, method, method == MP_METHOD_GAUSS_SEIDEL ? MP_FORM_FP64 : form))) return rc;
+            rc = method == MP_METHOD_SPARSE_CG      ? fe_solve_cg(ctx, st)
+                 : method == MP_METHOD_GAUSS_SEIDEL ? fe_solve_gs(ctx, st)
+                                                    : fe_solve_ldlt(ctx, form, st);
+            if (rc) return rc;
+            if ((rc = fe_update_d(ctx, &L2))) return rc;
+            if ((rc = fe_uh(ctx))) return rc;
+        }
+        ms_factor = st->ms_factor;
         st->newton_iterations = 1;
         st->l2 = L2;
-        if ((rc = fe_uh(ctx))) return rc;
     }
     cudaEventRecord(ctx->t0.b, ctx->stream);
     MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

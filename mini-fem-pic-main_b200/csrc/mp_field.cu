@@ -199,44 +199,48 @@ int fe_dense_j(mp_ctx *ctx) {
     return MP_OK;
 }
 
-// as_array = false: the solver at hand takes J = K - diag(FP) from the sparse K
-// and FP, and the dense array is formed only if something asks for it.
+// Before FP is formed for a J of the given method and form: an FP64 J that a
+// later solve may still use is not left without its FP.
+int fe_before_fp(mp_ctx *ctx, int method, int form) {
+    const bool fp64_j = ctx->K && method <= MP_METHOD_LAPACK && form == MP_FORM_FP64;
+    if (!fp64_j && ctx->j_current && !ctx->j_dense) return fe_dense_j(ctx);
+    return MP_OK;
+}
+
+// After it: what J the context now holds.  as_array = false: the solver at hand
+// takes J = K - diag(FP) from the sparse K and FP, and a dense array is formed
+// only if something asks for it.
+int fe_after_fp(mp_ctx *ctx, int method, int form, bool as_array) {
+    ctx->j32_current = false;
+    ctx->fp_is_j = false;
+    if (method == MP_METHOD_SPARSE_CG || method == MP_METHOD_SPARSE_NEWTON || !ctx->K) return MP_OK;
+    if (form == MP_FORM_MIXED) {
+        // the mixed form factors an FP32 copy and refines against K and FP: no FP64 J
+        if (!as_array) return MP_OK;
+        int rc = fe_j32_from_k(ctx);
+        if (rc) return rc;
+        ctx->j32_current = true;
+        return MP_OK;
+    }
+    ctx->j_dense = false;
+    ctx->j_current = true;
+    ctx->fp_is_j = true;
+    return as_array ? fe_dense_j(ctx) : MP_OK;
+}
+
 int fe_build_j(mp_ctx *ctx, int method, int form, bool as_array) {
     // the full symmetric J serves both dense solvers (Lapack reads only one
     // triangle); the sparse methods apply J = K - diag(FP) from K and FP
-    const bool fp64_j = ctx->K && method <= MP_METHOD_LAPACK && form == MP_FORM_FP64;
-    if (!fp64_j && ctx->j_current && !ctx->j_dense) {
-        // FP is about to change under an FP64 J that a later solve may still use
-        int rc = fe_dense_j(ctx);
-        if (rc) return rc;
-    }
+    int rc = fe_before_fp(ctx, method, form);
+    if (rc) return rc;
     int th = 256;
     k_node_terms<<<(ctx->n_nodes + th - 1) / th, th, 0, ctx->stream>>>(
         ctx->n_nodes, ctx->ID, nullptr, ctx->d, 0.0, -QE / EPS0, ctx->n0, ctx->phi0, ctx->kTe, 1 / ctx->kTe,
         nullptr, ctx->work), ++ctx->launches;
     k_eq_gather<<<(ctx->neq + th - 1) / th, th, 0, ctx->stream>>>(ctx->neq, ctx->eq_ptr, ctx->eq_tet, ctx->eq_a,
                                                                  ctx->detJ, ctx->work, ctx->FP, 0), ++ctx->launches;
-    if (method == MP_METHOD_SPARSE_CG || method == MP_METHOD_SPARSE_NEWTON || !ctx->K) {
-        ctx->j32_current = false;
-        ctx->fp_is_j = false;
-    } else if (form == MP_FORM_MIXED) {
-        // the mixed form factors an FP32 copy and refines against K and FP: no FP64 J
-        ctx->fp_is_j = false;
-        ctx->j32_current = false;
-        if (as_array) {
-            int rc = fe_j32_from_k(ctx);
-            if (rc) return rc;
-            ctx->j32_current = true;
-        }
-    } else {
-        ctx->j32_current = false;
-        ctx->j_dense = false;
-        ctx->j_current = true;
-        ctx->fp_is_j = true;
-        if (as_array) return fe_dense_j(ctx);
-    }
     MP_CUDA(ctx, cudaGetLastError());
-    return MP_OK;
+    return fe_after_fp(ctx, method, form, as_array);
 }
 
 // ---- d -= y ; L2 = sqrt(sum y^2)/neq (FESolver.cpp:341-349) ---------------------------

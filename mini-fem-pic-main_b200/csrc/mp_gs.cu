@@ -370,8 +370,9 @@ int gs_prepare(mp_ctx *ctx, bool *usable) {
     return MP_OK;
 }
 
-// Sweeps J y = G from the current y; FP is J's diagonal term.
-int gs_solve(mp_ctx *ctx, double tol, mp_newton_stats *st) {
+// Sweeps J y = G from the current y; FP is J's diagonal term.  *stop: a device word
+// that is not zero when the solve failed.
+int gs_enqueue(mp_ctx *ctx, double tol, const unsigned **stop) {
     GsState *s = static_cast<GsState *>(ctx->gs);
     GsArgs a = s->a;
     a.kval = ctx->sp_val;
@@ -398,12 +399,18 @@ int gs_solve(mp_ctx *ctx, double tol, mp_newton_stats *st) {
     ++ctx->launches;
     kt_end(ctx, mk);
     MP_CUDA(ctx, cudaMemcpyAsync(s->out_host, s->out, sizeof(double) * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (stop) *stop = reinterpret_cast<const unsigned *>(s->out + 3) + 1;  // the high word of 1.0
+    return MP_OK;
+}
+
+// The solve's results, after the stream has been waited for.
+int gs_finish(mp_ctx *ctx, mp_newton_stats *st) {
+    GsState *s = static_cast<GsState *>(ctx->gs);
     if (s->out_host[3] != 0.0) return fail(ctx, MP_ERR_TIMEOUT, "a bounded wait in the Gauss-Seidel sweep gave up");
     if (st) {
         const bool converged = s->out_host[2] != 0.0;
         st->linear_iterations = converged ? (int)s->out_host[0] - 1 : ctx->gs_max_sweeps;
-        st->linear_residual = std::sqrt(s->out_host[1]) / a.n;
+        st->linear_residual = std::sqrt(s->out_host[1]) / ctx->neq;
         if (!converged) st->linear_failures++;
     }
     return MP_OK;

@@ -186,6 +186,8 @@ struct mp_ctx {
     double *scal_host = nullptr;          // pinned
     int *eq_ptr = nullptr, *eq_tet = nullptr;   // CSR equation -> (tet, a) sorted by tet
     unsigned char *eq_a = nullptr;
+    int *eq_node = nullptr;               // equation -> node
+    bool one_node_each = false;           // ID numbers every equation exactly once
     double *gs_minv = nullptr;            // Gauss-Seidel: (D+L)^-1, [neq][neq]
     // sparse K, sliced ELLPACK (slices of 32 rows): entry k of row P (columns
     // ascending) at sp_ptr[P >> 5] + 32 * k + (P & 31); padding col = P, val = 0
@@ -254,16 +256,34 @@ int launch_compact(mp_ctx *ctx);
 int launch_convert_form(mp_ctx *ctx, int to_form);
 int launch_update_ef(mp_ctx *ctx);
 
+// A whole Newton step on the device (mp_newton.cu): F1, G and FP; the check of a
+// direct solve, deciding on the device whether its solution is taken; the update
+// of d and uh, unless *stop, with the step's scalars on their way to the host.
+struct NewtonState {
+    double l2, rn, bn;            // ||y|| / neq, ||G - J y||, ||G||
+    bool taken;
+    unsigned long long flags;
+};
+int newton_terms(mp_ctx *ctx, const double *den, bool clear_y, unsigned *clear, int clear_words);
+int newton_check(mp_ctx *ctx, double rtol, unsigned long long bad_flags);
+const unsigned *newton_go(mp_ctx *ctx);
+int newton_update(mp_ctx *ctx, const unsigned *stop);
+void newton_read(mp_ctx *ctx, NewtonState *s);
+
 int fe_build_f1(mp_ctx *ctx, const double *den_dev);
 int fe_residual(mp_ctx *ctx);
 int fe_build_j(mp_ctx *ctx, int method, int form = MP_FORM_FP64, bool as_array = true);
+int fe_before_fp(mp_ctx *ctx, int method, int form);
+int fe_after_fp(mp_ctx *ctx, int method, int form, bool as_array);
 int fe_dense_j(mp_ctx *ctx);
 int nd_prepare(mp_ctx *ctx, bool mixed, bool *usable);
-int nd_factor_solve(mp_ctx *ctx, const double *b, double *y);
+unsigned *nd_control(mp_ctx *ctx, int *words);
+int nd_factor_solve(mp_ctx *ctx, const double *b, double *y, bool control_cleared = false);
 int nd_solve_add(mp_ctx *ctx, const double *b, double *y);
 void nd_free(mp_ctx *ctx);
 int gs_prepare(mp_ctx *ctx, bool *usable);
-int gs_solve(mp_ctx *ctx, double tol, mp_newton_stats *st);
+int gs_enqueue(mp_ctx *ctx, double tol, const unsigned **stop);
+int gs_finish(mp_ctx *ctx, mp_newton_stats *st);
 void gs_free(mp_ctx *ctx);
 int fe_pattern_fits(mp_ctx *ctx, bool *fits);
 int fe_j32_from_k(mp_ctx *ctx);
@@ -281,6 +301,9 @@ int fe_sparse_from_host(mp_ctx *ctx, const double *const *rows, const double *de
 int fe_residual_sparse(mp_ctx *ctx);
 int fe_resid_j_sparse(mp_ctx *ctx, const double *y, const double *b, double *r, float *r32, double *sums);
 int fe_solve_cg(mp_ctx *ctx, mp_newton_stats *st);
+int cg_enqueue(mp_ctx *ctx, const unsigned **stop);
+int cg_finish(mp_ctx *ctx, mp_newton_stats *st);
+int fe_step_lean(mp_ctx *ctx, const double *den, int method, int form, bool first, mp_newton_stats *st, double *l2);
 void solve_free(mp_ctx *ctx);
 void adjoint_free(mp_ctx *ctx);
 void inject_free(mp_ctx *ctx);

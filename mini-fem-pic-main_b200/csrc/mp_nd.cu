@@ -1083,20 +1083,26 @@ static int nd_launch_solve(mp_ctx *ctx, NdState *s, bool back, const double *b, 
     return MP_OK;
 }
 
-static int nd_begin(mp_ctx *ctx, NdState *s) {
+static int nd_begin(mp_ctx *ctx, NdState *s, bool control_cleared) {
     if (s->epoch >= 0x7ffffff0u) {
         MP_CUDA(ctx, cudaMemsetAsync(s->flag, 0, sizeof(unsigned) * s->words, ctx->stream));
         s->epoch = 0;
     }
     s->epoch++;
-    MP_CUDA(ctx, cudaMemsetAsync(s->ctl, 0, sizeof(unsigned) * 8, ctx->stream));
+    if (!control_cleared) MP_CUDA(ctx, cudaMemsetAsync(s->ctl, 0, sizeof(unsigned) * 8, ctx->stream));
     return MP_OK;
 }
 
+// The words that have to be zero when a factorization starts.
+unsigned *nd_control(mp_ctx *ctx, int *words) {
+    *words = 8;
+    return state_of(ctx)->ctl;
+}
+
 // Factors J = K - diag(FP) and solves J y = b.
-int nd_factor_solve(mp_ctx *ctx, const double *b, double *y) {
+int nd_factor_solve(mp_ctx *ctx, const double *b, double *y, bool control_cleared) {
     NdState *s = state_of(ctx);
-    int rc = nd_begin(ctx, s);
+    int rc = nd_begin(ctx, s, control_cleared);
     if (rc) return rc;
     NdArgs a;
     a.task = s->task;
@@ -1127,7 +1133,7 @@ int nd_factor_solve(mp_ctx *ctx, const double *b, double *y) {
 // y += J^-1 b with the last factor.
 int nd_solve_add(mp_ctx *ctx, const double *b, double *y) {
     NdState *s = state_of(ctx);
-    int rc = nd_begin(ctx, s);
+    int rc = nd_begin(ctx, s, false);
     if (rc) return rc;
     if ((rc = nd_launch_solve(ctx, s, false, b, nullptr, false))) return rc;
     return nd_launch_solve(ctx, s, true, b, y, true);

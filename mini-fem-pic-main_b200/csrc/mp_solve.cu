@@ -150,6 +150,9 @@ static int ensure_scratch(mp_ctx *ctx, SolveScratch **out) {
 // residual stalls above 0.7 of the previous one): the FP64 factorization's
 // accuracy, so y matches dsysv_'s to the FP64 form's tolerance.
 constexpr double REFINE_RTOL = 1e-14;
+constexpr double GS_TOL = 1e-4;  // solveLinear's ||b - A x|| / neq, src/FESolver.cpp:564-590
+
+static int solve_dense(mp_ctx *ctx, int form, mp_newton_stats *st);
 
 // A residual above this share of ||G|| (an indefinite J can meet a bad pivot
 // order) sends the sparse factorization's solve to the dense one.
@@ -157,16 +160,20 @@ constexpr double SPARSE_RTOL = 1e-9;
 
 // The direct solve by the sparse factorization; *done is false when the dense
 // one has to take it over (a zero or non-finite pivot, a poor residual).
-static int solve_nd(mp_ctx *ctx, int form, mp_newton_stats *st, bool *done) {
+// enqueued: nd_factor_solve and newton_check have run, rn and bn hold their norms.
+static int solve_nd(mp_ctx *ctx, int form, mp_newton_stats *st, bool *done, bool enqueued, double rn, double bn) {
     *done = false;
-    cudaEventRecord(ctx->t1.a, ctx->stream);
-    int rc = nd_factor_solve(ctx, ctx->G, ctx->y);
-    if (rc) return rc;
-    cudaEventRecord(ctx->t1.b, ctx->stream);
-    double rn = 0, bn = 0, prev = 1e300;
+    int rc;
+    if (!enqueued) {
+        cudaEventRecord(ctx->t1.a, ctx->stream);
+        if ((rc = nd_factor_solve(ctx, ctx->G, ctx->y))) return rc;
+        cudaEventRecord(ctx->t1.b, ctx->stream);
+        if ((rc = resid_norms(ctx, ctx->y, ctx->G, ctx->work, nullptr, &rn, &bn))) return rc;
+    }
+    double prev = 1e300;
     int it = 1;
     for (; it < 60; it++) {
-        if ((rc = resid_norms(ctx, ctx->y, ctx->G, ctx->work, nullptr, &rn, &bn))) return rc;
+        if (it > 1 && (rc = resid_norms(ctx, ctx->y, ctx->G, ctx->work, nullptr, &rn, &bn))) return rc;
         if (form == MP_FORM_FP64 || !(rn > REFINE_RTOL * bn) || !(rn <= SPARSE_RTOL * bn) || rn > 0.7 * prev) break;
         prev = rn;
         if ((rc = nd_solve_add(ctx, ctx->work, ctx->y))) return rc;
@@ -187,6 +194,66 @@ static int solve_nd(mp_ctx *ctx, int form, mp_newton_stats *st, bool *done) {
     return MP_OK;
 }
 
+// One Newton step (F1, G, FP, the solve, the update of d and uh) by the method's
+// sparse solver, enqueued whole and read back once; *l2 = ||y|| / neq.  The
+// solver's plan is usable (nd_prepare, gs_prepare; conjugate gradients need none)
+// and every equation has its node.
+int fe_step_lean(mp_ctx *ctx, const double *den, int method, int form, bool first, mp_newton_stats *st, double *l2) {
+    const bool cg = method == MP_METHOD_SPARSE_CG || method == MP_METHOD_SPARSE_NEWTON;
+    const bool gs = method == MP_METHOD_GAUSS_SEIDEL || (method == MP_METHOD_NONLINEAR && form == MP_FORM_FP64);
+    const int jform = gs ? MP_FORM_FP64 : form;
+    int rc, words = 0;
+    unsigned *clear = cg || gs ? nullptr : nd_control(ctx, &words);
+    if ((rc = fe_before_fp(ctx, method, jform))) return rc;
+    if ((rc = newton_terms(ctx, den, first, clear, words))) return rc;
+    if ((rc = fe_after_fp(ctx, method, jform, false))) return rc;
+    const unsigned *stop = nullptr;
+    if (cg) {
+        if ((rc = cg_enqueue(ctx, &stop))) return rc;
+    } else if (gs) {
+        if ((rc = gs_enqueue(ctx, GS_TOL, &stop))) return rc;
+    } else {
+        cudaEventRecord(ctx->t1.a, ctx->stream);
+        if ((rc = nd_factor_solve(ctx, ctx->G, ctx->y, true))) return rc;
+        cudaEventRecord(ctx->t1.b, ctx->stream);
+        if ((rc = newton_check(ctx, form == MP_FORM_FP64 ? SPARSE_RTOL : REFINE_RTOL,
+                               FLAG_SINGULAR | FLAG_LOOKBACK_TIMEOUT)))
+            return rc;
+        stop = newton_go(ctx);
+    }
+    if ((rc = newton_update(ctx, stop))) return rc;
+    MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    NewtonState s;
+    newton_read(ctx, &s);
+    if (cg || gs) {
+        if ((rc = cg ? cg_finish(ctx, st) : gs_finish(ctx, st))) return rc;
+        *l2 = s.l2;
+        return MP_OK;
+    }
+    if (form == MP_FORM_FP64) ctx->j_current = false;  // one solve a build of J
+    if (s.taken) {
+        st->linear_iterations = 1;
+        st->linear_residual = s.rn / ctx->neq;
+        float ms = 0;
+        cudaEventElapsedTime(&ms, ctx->t1.a, ctx->t1.b);
+        st->ms_factor = ms;
+        *l2 = s.l2;
+        return MP_OK;
+    }
+    bool done = false;
+    if ((rc = solve_nd(ctx, form, st, &done, true, s.rn, s.bn))) return rc;
+    if (!done) {
+        if (form == MP_FORM_FP64) ctx->j_current = true;
+        if ((rc = solve_dense(ctx, form, st))) return rc;
+    }
+    MP_CUDA(ctx, cudaMemsetAsync(ctx->scal, 0, sizeof(double), ctx->stream));
+    if ((rc = newton_update(ctx, nullptr))) return rc;
+    MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    newton_read(ctx, &s);
+    *l2 = s.l2;
+    return MP_OK;
+}
+
 int fe_solve_ldlt(mp_ctx *ctx, int form, mp_newton_stats *st) {
     int rc;
     if (form == MP_FORM_FP64 && !ctx->j_current) return fail(ctx, MP_ERR_STATE, "no current FP64 J (build it first)");
@@ -195,12 +262,18 @@ int fe_solve_ldlt(mp_ctx *ctx, int form, mp_newton_stats *st) {
         (rc = nd_prepare(ctx, form == MP_FORM_MIXED, &nd)))
         return rc;
     if (nd) {
-        if ((rc = solve_nd(ctx, form, st, &nd))) return rc;
+        if ((rc = solve_nd(ctx, form, st, &nd, false, 0, 0))) return rc;
         if (nd) {
             if (form == MP_FORM_FP64) ctx->j_current = false;  // one solve a build of J
             return MP_OK;
         }
     }
+    return solve_dense(ctx, form, st);
+}
+
+// The direct solve by the dense factorization.
+static int solve_dense(mp_ctx *ctx, int form, mp_newton_stats *st) {
+    int rc;
     SolveScratch *sp = nullptr;
     rc = ensure_scratch(ctx, &sp);
     if (rc) return rc;
@@ -602,11 +675,15 @@ __global__ void k_gs_resid(int neq, long long ld, const double *__restrict__ A, 
 
 int fe_solve_gs(mp_ctx *ctx, mp_newton_stats *st) {
     if (!ctx->j_current) return fail(ctx, MP_ERR_STATE, "no current FP64 J (build it first)");
-    const double tol = 1e-4;
+    const double tol = GS_TOL;
     int rc;
     bool lean = false;
     if (ctx->fp_is_j && (rc = gs_prepare(ctx, &lean))) return rc;
-    if (lean) return gs_solve(ctx, tol, st);
+    if (lean) {
+        if ((rc = gs_enqueue(ctx, tol, nullptr))) return rc;
+        MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        return gs_finish(ctx, st);
+    }
     SolveScratch *sp = nullptr;
     rc = ensure_scratch(ctx, &sp);
     if (rc) return rc;

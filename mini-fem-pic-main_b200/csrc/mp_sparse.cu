@@ -689,9 +689,9 @@ cudaError_t launch_cg(const CgArgs &a, int nb, cudaStream_t stream) {
 // Rows are split in contiguous runs of rows_per_block (>= CG_THREADS) over at
 // most one block per SM; a thread keeps its rows' state in registers up to 4
 // rows (n <= 4 * 512 * SMs), in global memory beyond.
-int fe_solve_cg(mp_ctx *ctx, mp_newton_stats *st) {
+// *stop: a device word that is not zero when the solve failed.
+int cg_enqueue(mp_ctx *ctx, const unsigned **stop) {
     const int n = ctx->neq;
-    if (n <= 0) return MP_OK;
     SparseScratch *s = scratch_of(ctx);
     // one row a thread while the rows fit one block per SM: a thread's rows are
     // worked one after the other, which costs more than the longer grid-wide
@@ -750,7 +750,14 @@ int fe_solve_cg(mp_ctx *ctx, mp_newton_stats *st) {
     ++ctx->launches;
     MP_CUDA(ctx, cudaMemcpyAsync(s->out_host, s->out, sizeof(double) * 4, cudaMemcpyDeviceToHost, ctx->stream));
     MP_CUDA(ctx, cudaMemcpyAsync(s->out_host + 4, s->sync + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-    MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (stop) *stop = s->sync + 1;
+    return MP_OK;
+}
+
+// The solve's results, after the stream has been waited for.
+int cg_finish(mp_ctx *ctx, mp_newton_stats *st) {
+    SparseScratch *s = scratch_of(ctx);
+    const int n = ctx->neq;
     unsigned status;
     std::memcpy(&status, s->out_host + 4, sizeof(unsigned));
     ctx->cg_last_iterations = (int)s->out_host[0];
@@ -764,6 +771,13 @@ int fe_solve_cg(mp_ctx *ctx, mp_newton_stats *st) {
     if (status & CG_NOT_SPD) return fail(ctx, MP_ERR_SINGULAR, "conjugate gradients: J is not definite");
     if (status & CG_MAX_IT) return fail(ctx, MP_ERR_NOT_CONVERGED, "conjugate gradients: iteration limit reached");
     return MP_OK;
+}
+
+int fe_solve_cg(mp_ctx *ctx, mp_newton_stats *st) {
+    int rc = cg_enqueue(ctx, nullptr);
+    if (rc) return rc;
+    MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return cg_finish(ctx, st);
 }
 
 }  // namespace mp

@@ -141,3 +141,28 @@ def test_j_of_a_step(tmp_path):
     b = np.random.default_rng(1).normal(size=ctx.neq)
     ctx.solve_linear(mp.LAPACK, mp.FP64, b=b)
     assert rel(ctx.fe_get("y"), np.linalg.solve(J, b)) < TOL
+
+
+@pytest.mark.parametrize("n,sphere", [(2, False), (5, False), (8, False), (10, True)])
+@pytest.mark.parametrize("method", [mp.LAPACK, mp.GAUSS_SEIDEL, mp.SPARSE_CG])
+def test_step_terms_bitwise(tmp_path, n, sphere, method):
+    """The fused step's F1 and G are those of the separate entry points bit for bit,
+    and its update is d - y and g + d in one rounding each."""
+    kd, path = make_deck(tmp_path, n, sphere=(50.0, 50.0, 50.0, 20.0) if sphere else None)
+    dk = mp.Deck.load(path)
+    ctx = context(dk, sphere)
+    rng = np.random.default_rng(n)
+    den = 1e10 * (1 + 0.1 * rng.standard_normal(dk.mesh.n_nodes))
+    d, F1 = rng.normal(0.0, 0.5, ctx.neq), rng.normal(0.0, 1e-3, ctx.neq)
+    ctx.fe_set("d", d)
+    ctx.fe_set("F1", F1)
+    ctx.build_f1(den)
+    ctx.residual()
+    ref = ctx.fe_get("F1"), ctx.fe_get("G")
+    ctx.fe_set("F1", F1)
+    ctx.compute_phi(method, mp.FP64, ion_den=den)
+    assert np.array_equal(ctx.fe_get("F1"), ref[0]) and np.array_equal(ctx.fe_get("G"), ref[1])
+    ID = dk.mesh.fe_geometry()[0]
+    y, now, uh, g = (ctx.fe_get(k) for k in ("y", "d", "uh", "g"))
+    assert np.array_equal(now, d - y)
+    assert np.array_equal(uh, np.where(ID >= 0, g + now[ID], g))
