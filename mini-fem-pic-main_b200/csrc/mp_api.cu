@@ -161,10 +161,9 @@ static int ensure_dstage(mp_ctx *ctx, size_t bytes) {
     return MP_OK;
 }
 
-// Reads the counters back and turns error flags into a status.
-static int sync_counters(mp_ctx *ctx) {
-    MP_CUDA(ctx, cudaMemcpyAsync(ctx->counters_host, ctx->counters, sizeof(unsigned long long) * C_COUNT,
-                                 cudaMemcpyDeviceToHost, ctx->stream));
+// Waits for the stream and turns the host's copy of the counters, which the
+// last kernel or copy in the stream wrote, into counts and a status.
+static int read_counters(mp_ctx *ctx) {
     MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     ctx->n_host = (long long)ctx->counters_host[C_N];
     ctx->dead_host = (long long)ctx->counters_host[C_DEAD];
@@ -181,6 +180,13 @@ static int sync_counters(mp_ctx *ctx) {
         return fail(ctx, MP_ERR_WALK_LIMIT, "a particle's tet walk exceeded the hop limit");
     }
     return MP_OK;
+}
+
+// Reads the counters back.
+static int sync_counters(mp_ctx *ctx) {
+    MP_CUDA(ctx, cudaMemcpyAsync(ctx->counters_host, ctx->counters, sizeof(unsigned long long) * C_COUNT,
+                                 cudaMemcpyDeviceToHost, ctx->stream));
+    return read_counters(ctx);
 }
 
 }  // namespace mp
@@ -302,6 +308,7 @@ int mp_create(int device, const mp_mesh_desc *m, mp_ctx **out) {
     cudaMemsetAsync(ctx->ef, 0, sizeof(double) * 3 * nt, st);
     cudaMemsetAsync(ctx->den, 0, sizeof(double) * nn, st);
     cudaMemsetAsync(ctx->counters, 0, sizeof(unsigned long long) * C_COUNT, st);
+    cudaMemsetAsync(ctx->den_fixed, 0, sizeof(unsigned long long) * nn, st);
     upload_quadrature(st);
     cudaEventCreate(&ctx->t0.a); cudaEventCreate(&ctx->t0.b);
     cudaEventCreate(&ctx->t1.a); cudaEventCreate(&ctx->t1.b);
@@ -326,7 +333,7 @@ int mp_destroy(mp_ctx *ctx) {
     inject_free(ctx);
     sparse_free(ctx);
     void *dev[] = {ctx->tets, ctx->tets32, ctx->tet_x0, ctx->con, ctx->ef, ctx->node_volume, ctx->node_pos,
-                   ctx->den, ctx->den_fixed, ctx->counters, ctx->scal, ctx->compact_off, ctx->sort_hist,
+                   ctx->den, ctx->den_fixed, ctx->counters, ctx->scal, ctx->compact_off, ctx->sort_hist, ctx->scan_part,
                    ctx->part_block[0], ctx->part_block[1], ctx->ID, ctx->LM, ctx->detJ, ctx->nx, ctx->g, ctx->uh,
                    ctx->d, ctx->F0, ctx->F1, ctx->G, ctx->y, ctx->fvec, ctx->FP, ctx->work, ctx->K, ctx->J,
                    ctx->J32, ctx->K32, ctx->eq_ptr, ctx->eq_tet, ctx->eq_a, ctx->eq_node, ctx->gs_minv, ctx->den_in, ctx->dstage};
@@ -553,9 +560,11 @@ int mp_particles_download(mp_ctx *ctx, int64_t n_max, double *pos, int64_t pos_s
 int mp_push_scatter(mp_ctx *ctx, double q_over_m, double dt, double spwt, double *den_out, mp_step_stats *stats) {
     if (!ctx) return MP_ERR_ARG;
     long long n_before = ctx->n_host - ctx->dead_host;
-    cudaEventRecord(ctx->ts.a, ctx->stream);
     int rc;
+    bool sorted = false;
     if (ctx->sort_period > 0 && ++ctx->steps_since_sort >= ctx->sort_period) {
+        cudaEventRecord(ctx->ts.a, ctx->stream);
+        sorted = true;
         rc = launch_sort_by_tet(ctx);
         if (rc) return rc;
         ctx->steps_since_sort = 0;
@@ -568,7 +577,7 @@ int mp_push_scatter(mp_ctx *ctx, double q_over_m, double dt, double spwt, double
     if (den_out)
         MP_CUDA(ctx, cudaMemcpyAsync(den_out, ctx->den, sizeof(double) * ctx->n_nodes, cudaMemcpyDeviceToHost,
                                      ctx->stream));
-    rc = sync_counters(ctx);
+    rc = read_counters(ctx);  // k_normalise wrote the host's copy
     if (ctx->ktime_mask & (1u << MP_KT_PUSH)) {
         float ka = 0;
         if (cudaEventElapsedTime(&ka, ctx->tp.a, ctx->tp.b) == cudaSuccess) {
@@ -589,7 +598,7 @@ int mp_push_scatter(mp_ctx *ctx, double q_over_m, double dt, double spwt, double
         stats->lost = (int64_t)ctx->counters_host[C_LOST];
         float ka = 0, kb = 0;
         cudaEventElapsedTime(&ka, ctx->tp.a, ctx->tp.b);
-        cudaEventElapsedTime(&kb, ctx->ts.a, ctx->ts.b);
+        cudaEventElapsedTime(&kb, sorted ? ctx->ts.a : ctx->tp.a, ctx->ts.b);
         stats->ms_kernel = ka;
         stats->ms_step = kb;
     }

@@ -63,13 +63,14 @@ struct PartsF32 {
 enum Counter {
     C_N = 0,          // particle slots in use (live + holes)
     C_DEAD = 1,       // holes: slots of particles that left the domain
-    C_EXITS = 2,      // particles that left this push          } zeroed
-    C_HOPS = 3,       // total hops this push                   } before
-    C_MAX_HOPS = 4,   // longest walk this push                 } every
-    C_NEAR = 5,       // mixed form: FP64 near-face re-tests    } push
+    C_EXITS = 2,      // particles that left this push          } zero
+    C_HOPS = 3,       // total hops this push                   } between
+    C_MAX_HOPS = 4,   // longest walk this push                 } pushes (k_normalise)
+    C_NEAR = 5,       // mixed form: FP64 near-face re-tests    }
     C_FLAGS = 6,      // error bits (FLAG_*), cleared when reported
     C_NEXT_ID = 7,    // next particle id
-    C_LOST = 8,       // walks that hit the hop limit and were absorbed (zeroed before every push)
+    C_LOST = 8,       // walks that hit the hop limit and were absorbed (zero between pushes)
+    C_TICKET = 9,     // blocks done, of a kernel whose last block finishes up (zero between kernels)
     C_COUNT = 16
 };
 enum Flag : unsigned long long {
@@ -127,7 +128,7 @@ struct mp_ctx {
     int *con = nullptr;                   // [n_tets][4]
     double *den = nullptr;                // [n_nodes]
     double *den_in = nullptr;             // [n_nodes] host-supplied density for computePhi
-    unsigned long long *den_fixed = nullptr;  // [n_nodes] fixed-point accumulator
+    unsigned long long *den_fixed = nullptr;  // [n_nodes] the push's accumulator, fixed-point or FP64; zero between pushes
 
     // particles
     int form = MP_FORM_FP64;
@@ -153,7 +154,9 @@ struct mp_ctx {
     void *stage = nullptr;
     size_t stage_bytes = 0;
     // sort scratch
-    int *sort_hist = nullptr;
+    int *sort_hist = nullptr;             // [n_tets] counts, then cursors
+    int *scan_part = nullptr;             // totals of a scan's blocks, then their offsets
+    long long scan_part_len = 0;
     void *sort_tmp = nullptr;
 
     // FE
