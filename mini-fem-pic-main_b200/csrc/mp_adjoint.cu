@@ -28,6 +28,12 @@
 // at injection by vdbar += dir.vbar, Ebar[c0] -= 0.5*qm*dt*vbar.  Finally
 // phibar[n] = -sum over (e,a) with con[e][a] = n of NX[e][a].Ebar[e].
 // The tangent (forward mode) carries (dx, dv) along the same cells.
+//
+// The slots of one call to mp_adjoint_add_particles are laid out by cell: a
+// warp's slots start in a few tets and, with a common drift, stay near each
+// other, so the tet gathers hit the L1 and the lanes of one tet share their
+// atomics.  In the caller's order (at random over the box) every gather went to
+// the L2 and every slot-step took three atomics of its own.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -36,6 +42,7 @@
 
 #include "mp_internal.h"
 #include "mp_walk.cuh"
+#include "mp_warp.cuh"
 
 namespace mp {
 
@@ -72,7 +79,7 @@ struct AdjState {
     double *def = nullptr;      // [n_tets][3] tangent ef / reverse Ebar
     unsigned char *wall = nullptr;  // [n_tets] bit i: face opposite vertex i is a wall face
     double *nodes_a = nullptr, *nodes_b = nullptr;  // [n_nodes] scratch
-    double *scal = nullptr;     // device [4]: flux, vdbar, dflux, spare
+    double *scal = nullptr;     // device [4]: flux, vdbar, dflux, spare; [4]: slots by outcome (KIND_*), 64-bit counts
     double *scal_host = nullptr;
 };
 
@@ -216,40 +223,84 @@ __global__ void k_adj_wall(int n_tets, const TetRec *__restrict__ tets, const un
     wall[e] = m;
 }
 
+// This thread's slots [p, end), in steps of ADJ_THREADS: each CTA takes one
+// contiguous run of slots.  The loop's trip count is the same for a whole warp
+// (use p < a.n inside).
+#define ADJ_SLOTS(p)                                                                                        \
+    for (long long per_ = ((a.n + gridDim.x - 1) / gridDim.x + ADJ_THREADS - 1) / ADJ_THREADS * ADJ_THREADS, \
+                   p = blockIdx.x * per_ + threadIdx.x;                                                     \
+         p < (blockIdx.x + 1) * per_ && (p & ~31ll) < a.n; p += ADJ_THREADS)
+
+// Adds w[i] to out[con[i]] of the lanes' tets (on: whether this lane takes
+// part), the lanes of one tet together.  All lanes of the warp call it.
+__device__ __forceinline__ void add_to_nodes(bool on, int cell, const TetRec *tets, double (&w)[4], double *out) {
+    __syncwarp();
+    const int key = on ? cell : -2 - (int)(threadIdx.x & 31);
+    if (group_sum(key, w) && on) {
+        const int4 n = __ldg(reinterpret_cast<const int4 *>(tets[cell].con));
+        atomicAdd(&out[n.x], w[0]);
+        atomicAdd(&out[n.y], w[1]);
+        atomicAdd(&out[n.z], w[2]);
+        atomicAdd(&out[n.w], w[3]);
+    }
+}
+// The same for the three components of a per-tet vector.
+__device__ __forceinline__ void add_to_tet(bool on, int cell, double (&w)[3], double *out) {
+    const int key = on ? cell : -2 - (int)(threadIdx.x & 31);
+    if (group_sum(key, w) && on) {
+        atomicAdd(&out[3 * cell], w[0]);
+        atomicAdd(&out[3 * cell + 1], w[1]);
+        atomicAdd(&out[3 * cell + 2], w[2]);
+    }
+}
+
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_forward(AdjArgs a, double *den) {
     __shared__ double sh[ADJ_THREADS / 32];
+    __shared__ unsigned ended[4];
+    if (threadIdx.x < 4) ended[threadIdx.x] = 0;
+    __syncthreads();
     double flux = 0;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < a.n;
-         p += (long long)gridDim.x * blockDim.x) {
-        Slot s = start_slot(a, p);
-        const int k0 = a.first[p];
-        int kind = KIND_ALIVE, ek = a.K;
+    ADJ_SLOTS(p) {
+        const bool in = p < a.n;
+        int kind = KIND_ALIVE, ek = a.K, cell = -1;
         double lc[4] = {0, 0, 0, 0};
-        for (int k = k0; k < a.K; k++) {
-            if (k > k0 && k % a.C == 0) store_ck(a, k / a.C - 1, p, s);
-            kick_drift(s, a.ef, a.qm, a.dt);
-            kind = move_cell(a, s, k, p, lc);
-            if (kind != KIND_ALIVE) {
-                ek = k;
-                break;
+        if (in) {
+            Slot s = start_slot(a, p);
+            const int k0 = a.first[p];
+            for (int k = k0; k < a.K; k++) {
+                if (k > k0 && k % a.C == 0) store_ck(a, k / a.C - 1, p, s);
+                kick_drift(s, a.ef, a.qm, a.dt);
+                kind = move_cell(a, s, k, p, lc);
+                if (kind != KIND_ALIVE) {
+                    ek = k;
+                    break;
+                }
             }
+            if (kind == KIND_WALL) {
+                const double v2 =
+                    __dadd_rn(__dadd_rn(__dmul_rn(s.vx, s.vx), __dmul_rn(s.vy, s.vy)), __dmul_rn(s.vz, s.vz));
+                flux += __dmul_rn(a.spwt, __dmul_rn(0.5 * a.mass, v2));
+            } else if (kind == KIND_LIMIT) {
+                atomicOr(a.flags, FLAG_WALK_LIMIT);
+            } else if (kind == KIND_ALIVE && a.pinned) {
+                lambdas_fp64(a.tets + s.cell, s.x, s.y, s.z, lc);
+            }
+            if (kind == KIND_ALIVE) cell = s.cell;
+            a.exit_step[p] = ek;
+            a.kind[p] = (signed char)kind;
+            a.cell_end[p] = cell;
         }
-        if (kind == KIND_WALL) {
-            const double v2 = __dadd_rn(__dadd_rn(__dmul_rn(s.vx, s.vx), __dmul_rn(s.vy, s.vy)), __dmul_rn(s.vz, s.vz));
-            flux += __dmul_rn(a.spwt, __dmul_rn(0.5 * a.mass, v2));
-        } else if (kind == KIND_LIMIT) {
-            atomicOr(a.flags, FLAG_WALK_LIMIT);
-        } else if (kind == KIND_ALIVE) {
-            const TetRec *t = a.tets + s.cell;
-            if (a.pinned) lambdas_fp64(t, s.x, s.y, s.z, lc);
-            for (int i = 0; i < 4; i++) atomicAdd(&den[t->con[i]], lc[i]);
+        add_to_nodes(cell >= 0, cell, a.tets, lc, den);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const unsigned m = __ballot_sync(0xffffffffu, in && kind == q);
+            if (m && (threadIdx.x & 31) == 0) atomicAdd(&ended[q], __popc(m));
         }
-        a.exit_step[p] = ek;
-        a.kind[p] = (signed char)kind;
-        a.cell_end[p] = kind == KIND_ALIVE ? s.cell : -1;
     }
-    const double t = block_sum(flux, sh);
+    const double t = block_sum(flux, sh);  // a block barrier: ended[] is complete
     if (threadIdx.x == 0 && t != 0) atomicAdd(&a.scal[0], t);
+    if (threadIdx.x < 4 && ended[threadIdx.x])
+        atomicAdd(reinterpret_cast<unsigned long long *>(a.scal + 4) + threadIdx.x, (unsigned long long)ended[threadIdx.x]);
 }
 
 // den_out[n] = den[n] * (spwt / Vnode[n])   (the normalisation of MoveParticles)
@@ -264,14 +315,14 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_reverse(AdjArgs a, const do
                                                               double *ebar) {
     __shared__ double sh[ADJ_THREADS / 32];
     double vdbar = 0;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < a.n;
-         p += (long long)gridDim.x * blockDim.x) {
-        const int kind = a.kind[p];
-        if (kind != KIND_ALIVE && kind != KIND_WALL) continue;  // outputs do not depend on this slot
-        const int k0 = a.first[p];
-        const int last = kind == KIND_WALL ? a.exit_step[p] : a.K - 1;
+    ADJ_SLOTS(p) {
+        const int kind = p < a.n ? a.kind[p] : KIND_OTHER;
+        // the outputs depend only on slots that are inside at the end or left through the wall
+        const bool on = kind == KIND_ALIVE || kind == KIND_WALL;
+        const int k0 = on ? a.first[p] : 0;
+        const int last = on ? (kind == KIND_WALL ? a.exit_step[p] : a.K - 1) : -1;
         double xb[3] = {0, 0, 0}, vb[3] = {0, 0, 0};
-        if (kind == KIND_ALIVE) {
+        if (on && kind == KIND_ALIVE) {
             const TetRec *t = a.tets + a.cell_end[p];
             for (int i = 0; i < 4; i++) {
                 const int nd = t->con[i];
@@ -281,42 +332,58 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_reverse(AdjArgs a, const do
                 for (int d = 0; d < 3; d++) xb[d] += w * g[d];
             }
         }
+        // the segments of any of the warp's slots
+        const int j1 = __reduce_max_sync(0xffffffffu, on ? last / a.C : -1);
+        const int j0 = __reduce_min_sync(0xffffffffu, on ? k0 / a.C : 1 << 30);
         int cs[ADJ_MAX_SEGMENT];
-        for (int j = last / a.C; j >= k0 / a.C; j--) {
+        for (int j = j1; j >= j0; j--) {
             const int s0 = j * a.C;
             const int kb = s0 > k0 ? s0 : k0;
-            const int ke = s0 + a.C - 1 < last ? s0 + a.C - 1 : last;
-            Slot s = kb == k0 ? start_slot(a, p) : load_ck(a, j - 1, p);
-            double lc[4];
-            for (int k = kb; k <= ke; k++) {
-                cs[k - s0] = s.cell;
-                kick_drift(s, a.ef, a.qm, a.dt);
-                if (k == last) {
-                    if (kind == KIND_WALL) {
-                        const double c = fbar * a.spwt * a.mass;
-                        vb[0] = c * s.vx;
-                        vb[1] = c * s.vy;
-                        vb[2] = c * s.vz;
+            const int ke = s0 + a.C - 1 < last ? s0 + a.C - 1 : last;  // below kb: no step of this segment
+            if (on && kb <= ke) {
+                Slot s = kb == k0 ? start_slot(a, p) : load_ck(a, j - 1, p);
+                double lc[4];
+                for (int k = kb; k <= ke; k++) {
+                    cs[k - s0] = s.cell;
+                    kick_drift(s, a.ef, a.qm, a.dt);
+                    if (k == last) {
+                        if (kind == KIND_WALL) {
+                            const double c = fbar * a.spwt * a.mass;
+                            vb[0] = c * s.vx;
+                            vb[1] = c * s.vy;
+                            vb[2] = c * s.vz;
+                        }
+                    } else if (k < ke) {
+                        move_cell(a, s, k, p, lc);
                     }
-                } else if (k < ke) {
-                    move_cell(a, s, k, p, lc);
                 }
             }
-            for (int k = ke; k >= kb; k--) {
-                const int c = cs[k - s0];
+            __syncwarp();
+            for (int k = s0 + a.C - 1; k >= s0; k--) {
+                const bool step = on && k >= kb && k <= ke;
+                double w[3] = {0, 0, 0};
+                int c = 0;
+                if (step) {
+                    c = cs[k - s0];
 #pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    vb[d] += a.dt * xb[d];
-                    atomicAdd(&ebar[3 * c + d], a.qm * a.dt * vb[d]);
+                    for (int d = 0; d < 3; d++) {
+                        vb[d] += a.dt * xb[d];
+                        w[d] = a.qm * a.dt * vb[d];
+                    }
                 }
+                add_to_tet(step, c, w, ebar);
             }
         }
-        if (a.inj[p]) {
+        const bool injected = on && a.inj[p];
+        double w[3] = {0, 0, 0};
+        int c = 0;
+        if (injected) {
             vdbar += a.dir0 * vb[0] + a.dir1 * vb[1] + a.dir2 * vb[2];
-            const int c = a.cell0[p];
+            c = a.cell0[p];
 #pragma unroll
-            for (int d = 0; d < 3; d++) atomicAdd(&ebar[3 * c + d], -(a.qm * (0.5 * a.dt)) * vb[d]);
+            for (int d = 0; d < 3; d++) w[d] = -(a.qm * (0.5 * a.dt)) * vb[d];
         }
+        if (__any_sync(0xffffffffu, injected)) add_to_tet(injected, c, w, ebar);
     }
     const double t = block_sum(vdbar, sh);
     if (threadIdx.x == 0 && t != 0) atomicAdd(&a.scal[1], t);
@@ -340,42 +407,61 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_tangent(AdjArgs a, const do
                                                               double *dden) {
     __shared__ double sh[ADJ_THREADS / 32];
     double dflux = 0;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < a.n;
-         p += (long long)gridDim.x * blockDim.x) {
-        if (a.kind[p] == KIND_OTHER || a.kind[p] == KIND_LIMIT) continue;
-        Slot s = start_slot(a, p);
-        const int k0 = a.first[p];
-        double dx[3] = {0, 0, 0}, dv[3] = {0, 0, 0};
-        if (a.inj[p]) {
-            const double *de = def + 3 * s.cell;
-            const double dir[3] = {a.dir0, a.dir1, a.dir2};
-            for (int d = 0; d < 3; d++) dv[d] = dir[d] * dvd - a.qm * de[d] * (0.5 * a.dt);
-        }
-        int kind = KIND_ALIVE;
-        double lc[4];
-        for (int k = k0; k < a.K; k++) {
-            const double *de = def + 3 * s.cell;
-            for (int d = 0; d < 3; d++) {
-                dv[d] += a.qm * de[d] * a.dt;
-                dx[d] += dv[d] * a.dt;
+    ADJ_SLOTS(p) {
+        const bool on = p < a.n && a.kind[p] != KIND_OTHER && a.kind[p] != KIND_LIMIT;
+        int cell = -1;
+        double w[4] = {0, 0, 0, 0};
+        if (on) {
+            Slot s = start_slot(a, p);
+            const int k0 = a.first[p];
+            double dx[3] = {0, 0, 0}, dv[3] = {0, 0, 0};
+            if (a.inj[p]) {
+                const double *de = def + 3 * s.cell;
+                const double dir[3] = {a.dir0, a.dir1, a.dir2};
+                for (int d = 0; d < 3; d++) dv[d] = dir[d] * dvd - a.qm * de[d] * (0.5 * a.dt);
             }
-            kick_drift(s, a.ef, a.qm, a.dt);
-            kind = move_cell(a, s, k, p, lc);
-            if (kind != KIND_ALIVE) break;
-        }
-        if (kind == KIND_WALL) {
-            dflux += a.spwt * a.mass * (s.vx * dv[0] + s.vy * dv[1] + s.vz * dv[2]);
-        } else if (kind == KIND_ALIVE) {
-            const TetRec *t = a.tets + s.cell;
-            for (int i = 0; i < 4; i++) {
-                double g[3];
-                grad_lambda(t, i, g);
-                atomicAdd(&dden[t->con[i]], g[0] * dx[0] + g[1] * dx[1] + g[2] * dx[2]);
+            int kind = KIND_ALIVE;
+            double lc[4];
+            for (int k = k0; k < a.K; k++) {
+                const double *de = def + 3 * s.cell;
+                for (int d = 0; d < 3; d++) {
+                    dv[d] += a.qm * de[d] * a.dt;
+                    dx[d] += dv[d] * a.dt;
+                }
+                kick_drift(s, a.ef, a.qm, a.dt);
+                kind = move_cell(a, s, k, p, lc);
+                if (kind != KIND_ALIVE) break;
+            }
+            if (kind == KIND_WALL) {
+                dflux += a.spwt * a.mass * (s.vx * dv[0] + s.vy * dv[1] + s.vz * dv[2]);
+            } else if (kind == KIND_ALIVE) {
+                cell = s.cell;
+                for (int i = 0; i < 4; i++) {
+                    double g[3];
+                    grad_lambda(a.tets + cell, i, g);
+                    w[i] = g[0] * dx[0] + g[1] * dx[1] + g[2] * dx[2];
+                }
             }
         }
+        add_to_nodes(cell >= 0, cell, a.tets, w, dden);
     }
     const double t = block_sum(dflux, sh);
     if (threadIdx.x == 0 && t != 0) atomicAdd(&a.scal[2], t);
+}
+
+// Slots s0 + i <- particle order[i] of the packed arrays pos, vel [n][3].
+__global__ void k_adj_place(long long n, const double *__restrict__ pos, const double *__restrict__ vel,
+                            const int *__restrict__ cell, const int *__restrict__ order, int first, unsigned char inj,
+                            long long s0, double *px, double *py, double *pz, double *vx, double *vy, double *vz,
+                            int *cell0, int *firsts, unsigned char *injs) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const long long q = order[i], o = s0 + i;
+    px[o] = pos[3 * q]; py[o] = pos[3 * q + 1]; pz[o] = pos[3 * q + 2];
+    vx[o] = vel[3 * q]; vy[o] = vel[3 * q + 1]; vz[o] = vel[3 * q + 2];
+    cell0[o] = cell[q];
+    firsts[o] = first;
+    injs[o] = inj;
 }
 
 static AdjState *state(mp_ctx *ctx) { return reinterpret_cast<AdjState *>(ctx->adjoint); }
@@ -514,8 +600,8 @@ int mp_adjoint_setup(mp_ctx *ctx, int32_t steps, int32_t checkpoint_every, doubl
     MP_CUDA(ctx, cudaMalloc(&s->wall, nt));
     MP_CUDA(ctx, cudaMalloc(&s->nodes_a, sizeof(double) * nn));
     MP_CUDA(ctx, cudaMalloc(&s->nodes_b, sizeof(double) * nn));
-    MP_CUDA(ctx, cudaMalloc(&s->scal, sizeof(double) * 4));
-    MP_CUDA(ctx, cudaMallocHost(&s->scal_host, sizeof(double) * 4));
+    MP_CUDA(ctx, cudaMalloc(&s->scal, sizeof(double) * 8));
+    MP_CUDA(ctx, cudaMallocHost(&s->scal_host, sizeof(double) * 8));
     unsigned char *wn = nullptr;
     MP_CUDA(ctx, cudaMalloc(&wn, nn));
     MP_CUDA(ctx, cudaMemcpyAsync(wn, wall_nodes, nn, cudaMemcpyDefault, ctx->stream));
@@ -532,30 +618,30 @@ int mp_adjoint_add_particles(mp_ctx *ctx, int32_t first_step, int injected, int6
     if (!ctx || !s) return ctx ? fail(ctx, MP_ERR_STATE, "no adjoint setup") : MP_ERR_ARG;
     if (n < 0 || first_step < 0 || first_step >= s->K || (n > 0 && (!pos || !vel || !cell))) return MP_ERR_ARG;
     if (n == 0) return MP_OK;
-    std::vector<double> soa(6 * (size_t)n);
-    std::vector<int> c(n), f(n, first_step);
-    std::vector<unsigned char> in(n, injected ? 1 : 0);
-    // pos/vel may be host or device memory: stage through the host
-    std::vector<double> p3(3 * (size_t)n), v3(3 * (size_t)n);
-    MP_CUDA(ctx, cudaMemcpy(p3.data(), pos, sizeof(double) * 3 * n, cudaMemcpyDefault));
-    MP_CUDA(ctx, cudaMemcpy(v3.data(), vel, sizeof(double) * 3 * n, cudaMemcpyDefault));
+    if (n > (1ll << 31) - 1) return fail(ctx, MP_ERR_ARG, "more than 2^31 - 1 adjoint particles in one call");
+    // pos, vel and cell may be host or device memory; the slots' order by cell is made on the host
+    std::vector<int> c(n), order(n), at(ctx->n_tets + 1, 0);
     MP_CUDA(ctx, cudaMemcpy(c.data(), cell, sizeof(int) * n, cudaMemcpyDefault));
     for (int64_t i = 0; i < n; i++) {
         if (c[i] < 0 || c[i] >= ctx->n_tets) return fail(ctx, MP_ERR_ARG, "adjoint particle cell out of range");
-        for (int d = 0; d < 3; d++) {
-            soa[d * n + i] = p3[3 * i + d];
-            soa[(3 + d) * n + i] = v3[3 * i + d];
-        }
+        at[c[i] + 1]++;
     }
+    for (int t = 0; t < ctx->n_tets; t++) at[t + 1] += at[t];
+    for (int64_t i = 0; i < n; i++) order[at[c[i]]++] = (int)i;
     int rc = grow_slots(ctx, s, s->n + n);
     if (rc) return rc;
-    double *dst[6] = {s->px, s->py, s->pz, s->vx, s->vy, s->vz};
-    for (int d = 0; d < 6; d++)
-        MP_CUDA(ctx, cudaMemcpyAsync(dst[d] + s->n, soa.data() + d * n, sizeof(double) * n, cudaMemcpyHostToDevice,
-                                     ctx->stream));
-    MP_CUDA(ctx, cudaMemcpyAsync(s->cell0 + s->n, c.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
-    MP_CUDA(ctx, cudaMemcpyAsync(s->first + s->n, f.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
-    MP_CUDA(ctx, cudaMemcpyAsync(s->inj + s->n, in.data(), n, cudaMemcpyHostToDevice, ctx->stream));
+    if ((rc = ensure_dstage(ctx, (6 * sizeof(double) + 2 * sizeof(int)) * n))) return rc;
+    double *p3 = (double *)ctx->dstage, *v3 = p3 + 3 * n;
+    int *dc = (int *)(v3 + 3 * n), *dord = dc + n;
+    MP_CUDA(ctx, cudaMemcpyAsync(p3, pos, sizeof(double) * 3 * n, cudaMemcpyDefault, ctx->stream));
+    MP_CUDA(ctx, cudaMemcpyAsync(v3, vel, sizeof(double) * 3 * n, cudaMemcpyDefault, ctx->stream));
+    MP_CUDA(ctx, cudaMemcpyAsync(dc, c.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
+    MP_CUDA(ctx, cudaMemcpyAsync(dord, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
+    k_adj_place<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(
+        n, p3, v3, dc, dord, first_step, injected ? 1 : 0, s->n, s->px, s->py, s->pz, s->vx, s->vy, s->vz, s->cell0,
+        s->first, s->inj),
+        ++ctx->launches;
+    MP_CUDA(ctx, cudaGetLastError());
     MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     s->n += n;
     s->tape = false;
@@ -575,7 +661,7 @@ int mp_adjoint_forward(mp_ctx *ctx, const double *phi, double v_drift, int mode,
     MP_CUDA(ctx, cudaMemcpyAsync(s->nodes_b, phi, sizeof(double) * nn, cudaMemcpyDefault, ctx->stream));
     k_adj_ef<<<(nt + 255) / 256, 256, 0, ctx->stream>>>(nt, ctx->con, s->nx, s->nodes_b, s->ef), ++ctx->launches;
     MP_CUDA(ctx, cudaMemsetAsync(s->nodes_a, 0, sizeof(double) * nn, ctx->stream));
-    MP_CUDA(ctx, cudaMemsetAsync(s->scal, 0, sizeof(double) * 4, ctx->stream));
+    MP_CUDA(ctx, cudaMemsetAsync(s->scal, 0, sizeof(double) * 8, ctx->stream));
     s->vd = v_drift;
     const bool pinned = mode == MP_ADJ_PINNED;
     const bool record = s->record && !pinned;
@@ -587,7 +673,7 @@ int mp_adjoint_forward(mp_ctx *ctx, const double *phi, double v_drift, int mode,
     MP_CUDA(ctx, cudaGetLastError());
     cudaEventRecord(ctx->t0.b, ctx->stream);
     if (den_out) MP_CUDA(ctx, cudaMemcpyAsync(den_out, s->nodes_b, sizeof(double) * nn, cudaMemcpyDefault, ctx->stream));
-    MP_CUDA(ctx, cudaMemcpyAsync(s->scal_host, s->scal, sizeof(double) * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    MP_CUDA(ctx, cudaMemcpyAsync(s->scal_host, s->scal, sizeof(double) * 8, cudaMemcpyDeviceToHost, ctx->stream));
     MP_CUDA(ctx, cudaMemcpyAsync(ctx->counters_host + C_FLAGS, ctx->counters + C_FLAGS, sizeof(unsigned long long),
                                  cudaMemcpyDeviceToHost, ctx->stream));
     MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -596,14 +682,12 @@ int mp_adjoint_forward(mp_ctx *ctx, const double *phi, double v_drift, int mode,
     if (record) s->path_valid = true;
     if (st) {
         std::memset(st, 0, sizeof(*st));
-        std::vector<signed char> kind(s->n);
-        if (s->n) MP_CUDA(ctx, cudaMemcpy(kind.data(), s->kind, s->n, cudaMemcpyDeviceToHost));
+        unsigned long long ended[4];
+        std::memcpy(ended, s->scal_host + 4, sizeof(ended));
         st->slots = s->n;
-        for (signed char k : kind) {
-            if (k == KIND_ALIVE) st->alive++;
-            else if (k == KIND_WALL) st->wall_exits++;
-            else if (k == KIND_OTHER) st->other_exits++;
-        }
+        st->alive = (int64_t)ended[KIND_ALIVE];
+        st->wall_exits = (int64_t)ended[KIND_WALL];
+        st->other_exits = (int64_t)ended[KIND_OTHER];
         st->flux = s->scal_host[0];
         float ms = 0;
         cudaEventElapsedTime(&ms, ctx->t0.a, ctx->t0.b);

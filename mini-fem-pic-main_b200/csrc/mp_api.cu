@@ -149,7 +149,7 @@ static int ensure_stage(mp_ctx *ctx, size_t bytes) {
 }
 
 // Device staging of host appends and downloads, owned by the context.
-static int ensure_dstage(mp_ctx *ctx, size_t bytes) {
+int ensure_dstage(mp_ctx *ctx, size_t bytes) {
     if (bytes <= ctx->dstage_bytes) return MP_OK;
     MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if (ctx->dstage) cudaFree(ctx->dstage);

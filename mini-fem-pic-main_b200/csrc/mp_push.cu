@@ -14,6 +14,7 @@
 
 #include "mp_internal.h"
 #include "mp_walk.cuh"
+#include "mp_warp.cuh"
 
 namespace mp {
 
@@ -76,44 +77,6 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
-}
-
-// Sums v[0..3] over the lanes that share `key` (one tet), leaving the sums in
-// the group's lowest lane.  All 32 lanes must call it.  Returns true for the
-// lanes that hold a group sum.
-//
-// Pointer jumping over each group's member list: every lane starts pointing at
-// the next member above it and holds the sum of the members from itself up to
-// (not including) the one it points at; each round adds the pointed-to
-// lane's partial sum and takes over its pointer, so ceil(log2(group size))
-// rounds leave the whole group's sum in its lowest lane.  A round is one vote,
-// nine shuffles and four adds, and groups need not be contiguous (particles
-// that hopped since the last tet sort sit between their tet's others).  This
-// replaced a tree over group ranks that located the rank r + s member with a
-// bit search each round: FP64 push 0.0905 -> 0.0868 ms, mixed 0.0660 ->
-// 0.0592 ms on 2M ions sorted every 10 steps.  Summing runs of adjacent equal
-// keys instead (no match) was slower (0.14 ms): a tet's lanes split into
-// several runs once particles hop, and every run issues its own atomics.
-template <typename T>
-__device__ __forceinline__ bool group_sum4(int key, T v[4]) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const unsigned peers = __match_any_sync(FULL, key);
-    const unsigned above = peers & (0xfffffffeu << lane);  // members above this lane
-    int nxt = above ? __ffs(above) - 1 : -1;
-    while (__any_sync(FULL, nxt >= 0)) {
-        const int src = nxt >= 0 ? nxt : lane;
-        T t[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) t[i] = __shfl_sync(FULL, v[i], src);
-        const int n2 = __shfl_sync(FULL, nxt, src);
-        if (nxt >= 0) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) v[i] += t[i];
-            nxt = n2;
-        }
-    }
-    return (peers & ((1u << lane) - 1u)) == 0;
 }
 
 // Asynchronous global -> shared copies (cp.async, L2 only) for staging the
@@ -193,7 +156,7 @@ __device__ __forceinline__ void scatter_warp(int state, int cell, const int con[
 #pragma unroll
         for (int i = 0; i < 4; i++)
             q[i] = state == 1 ? (unsigned long long)__double2ll_rn((double)lcv[i] * FIXED_SCALE) : 0ull;
-        bool leader = group_sum4<unsigned long long>(key, q);
+        bool leader = group_sum(key, q);
         if (leader && state == 1) {
 #pragma unroll
             for (int i = 0; i < 4; i++) atomicAdd(&den_fixed[con[i]], q[i]);
@@ -202,7 +165,7 @@ __device__ __forceinline__ void scatter_warp(int state, int cell, const int con[
         double sv[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) sv[i] = state == 1 ? (double)lcv[i] : 0.0;
-        bool leader = group_sum4<double>(key, sv);
+        bool leader = group_sum(key, sv);
         if (leader && state == 1) {
 #pragma unroll
             for (int i = 0; i < 4; i++) atomicAdd(&den[con[i]], sv[i]);
