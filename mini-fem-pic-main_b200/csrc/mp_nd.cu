@@ -7,19 +7,20 @@
 // to run.  A tile is announced by its flag word; a task waits only for tiles
 // of tasks before it in the order, whose CTAs already run, so no co-residency
 // is assumed.
-//   warp 8 (one lane)  producer: takes the ticket, waits for the flags of a
+//   warp 16 (one lane) producer: takes the ticket, waits for the flags of a
 //                      product's two tiles and copies them (cp.async.bulk) into
 //                      one of two shared-memory stages, ahead of the others;
-//   warps 0-7          C -= A D B^T on the FP64 tensor cores (mma.sync m8n8k4),
+//   warps 0-15         C -= A D B^T on the FP64 tensor cores (mma.sync m8n8k4),
 //                      then the tile's end: off the diagonal L = C L_jj^-T D_j^-1;
 //                      on it the 64 x 64 factor, its inverse, and the forward
 //                      substitution of the right-hand side.
-//   warp 9 (one lane)  publisher: releases a finished tile's flag, so that only
+//   warp 17 (one lane) publisher: releases a finished tile's flag, so that only
 //                      it waits for the tile's stores.
 // Measured (B200, Newton step of the Lapack method, dense LDL^T before -> now): 567
-// unknowns 0.71 -> 0.23 ms, 8,379 15.6 -> 0.60 ms, 32,244 (mixed form) 41.4 ->
-// 1.46 ms.  The chain of diagonal blocks, 17.7 us a block (64 x 64 factor 8.9,
-// products through the tile before it 5, hand-over between SMs 2), bounds the
+// unknowns 0.71 -> 0.16 ms, 8,379 15.6 -> 0.48 ms, 32,244 (mixed form) 41.4 ->
+// 1.33 ms.  The chain of diagonal blocks, 15 us a block (64 x 64 factor 8.4,
+// products through the tile before it 3, hand-over between SMs 2; with 8 working
+// warps instead of 16, 17.7 us), bounds the
 // small meshes and the upper levels of the large ones; the FP64 tensor cores'
 // rate (64 multiply-adds a cycle and SM) and the tasks' own latency the lower levels.
 #include <algorithm>
@@ -36,7 +37,7 @@ namespace {
 constexpr int T = ND_TILE;
 constexpr int TT = T * T;
 constexpr int STAGES = 2;
-constexpr int WORK = 256;              // threads of warps 0-7
+constexpr int WORK = 512;              // threads of warps 0-15
 constexpr int THREADS = WORK + 64;     // and the producer's and the publisher's warp
 constexpr int PUBS = 4;
 constexpr unsigned POLL_LIMIT = 1u << 22;
@@ -64,6 +65,7 @@ struct Smem {
     double invt[7 * 7 * 64];           // its first 56 rows and columns, transposed
     double tt[7 * 64];                 // 8 rows of L times the inverse's rows above, transposed
     double r[T], d[T], dinv[T];
+    double z7[8][8];                   // by inverse block: the last 8 rows of z
     NdTask task[STAGES];
     NdItem item[STAGES];
     int last[STAGES];                  // 1: the task's last item, 2: no more tasks
@@ -137,15 +139,17 @@ __device__ bool poll(const unsigned *f, unsigned epoch, unsigned *ctl_abort, uns
         }
     }
 }
-// barrier of warps 0-7, and the same with a vote
-__device__ __forceinline__ void sync_work() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(WORK) : "memory"); }
+// barrier of the first N threads, and the same with a vote
+template <int N = WORK>
+__device__ __forceinline__ void sync_work() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(N) : "memory"); }
+template <int N = WORK>
 __device__ __forceinline__ bool all_work(bool p) {
     unsigned r;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 2, %2, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(r)
-        : "r"((unsigned)p), "n"(WORK)
+        : "r"((unsigned)p), "n"(N)
         : "memory");
     return r != 0;
 }
@@ -186,14 +190,13 @@ __device__ __forceinline__ double2 frag(const double *blk, int lane) {
     return *reinterpret_cast<const double2 *>(blk + 2 * lane);
 }
 
-// A warp's 8 x 8 blocks of a tile: rows h, h + 2, h + 4, h + 6 (h = warp / 4) and
-// two columns, {q, q + 4} or, for h = 1, {3 - q, 7 - q} (q = warp % 4, the SM
-// quarter it runs on), so that every quarter gets its share of a tile's leading
-// rows and columns (a part's last tile is rarely full) and of a triangular
-// product.
+// A warp's 8 x 8 blocks of a tile: rows h, h + 4 (h = warp / 4) and two columns,
+// {q, q + 4} or, for odd h, {3 - q, 7 - q} (q = warp % 4, the SM quarter it runs
+// on), so that every quarter gets its share of a tile's leading rows and columns
+// (a part's last tile is rarely full) and of a triangular product.
 struct TileBlocks {
     int h, c0;
-    __device__ __forceinline__ int row(int i) const { return h + 2 * i; }
+    __device__ __forceinline__ int row(int i) const { return h + 4 * i; }
     __device__ __forceinline__ int col(int j) const { return c0 + 4 * j; }
     __device__ __forceinline__ int at(int i, int j) const { return col(j) * 512 + row(i) * 64; }
 };
@@ -202,7 +205,7 @@ struct TileBlocks {
 // columns (J0 on), B scaled by d[].  No branches between the products: mma.sync
 // under a branch the compiler cannot prove uniform costs it a re-convergence.
 template <bool SCALE, int NI, int J0, int NJ>
-__device__ __forceinline__ void gemm_step(double (&acc)[4][2][2], const double *A, const double *B, const double *d,
+__device__ __forceinline__ void gemm_step(double (&acc)[2][2][2], const double *A, const double *B, const double *d,
                                           int k, const TileBlocks &tb, int lane) {
     double2 a[NI], b[2];
 #pragma unroll
@@ -227,23 +230,26 @@ __device__ __forceinline__ void gemm_step(double (&acc)[4][2][2], const double *
         for (int j = J0; j < J0 + NJ; j++) dmma(acc[i][j], a[i].y, b[j].y);
 }
 template <bool SCALE, int NI>
-__device__ __forceinline__ void gemm_rows(double (&acc)[4][2][2], const double *A, const double *B, const double *d,
+__device__ __forceinline__ void gemm_rows(double (&acc)[2][2][2], const double *A, const double *B, const double *d,
                                           int kb, bool two, const TileBlocks &tb, int lane) {
     if (SCALE) {
         if (two) {
-#pragma unroll 2
+#pragma unroll 1
             for (int k = 0; k < kb; k++) gemm_step<SCALE, NI, 0, 2>(acc, A, B, d, k, tb, lane);
         } else {
-#pragma unroll 2
+#pragma unroll 1
             for (int k = 0; k < kb; k++) gemm_step<SCALE, NI, 0, 1>(acc, A, B, d, k, tb, lane);
         }
     } else {
         // B lower triangular: block column k meets its block rows from k on
         const int k0 = min(kb, tb.col(0) + 1), k1 = min(kb, tb.col(1) + 1);
         if (two) {
+#pragma unroll 1
             for (int k = 0; k < k0; k++) gemm_step<SCALE, NI, 0, 2>(acc, A, B, d, k, tb, lane);
+#pragma unroll 1
             for (int k = k0; k < k1; k++) gemm_step<SCALE, NI, 1, 1>(acc, A, B, d, k, tb, lane);
         } else {
+#pragma unroll 1
             for (int k = 0; k < k0; k++) gemm_step<SCALE, NI, 0, 1>(acc, A, B, d, k, tb, lane);
         }
     }
@@ -251,63 +257,65 @@ __device__ __forceinline__ void gemm_rows(double (&acc)[4][2][2], const double *
 // acc += A B^T over kb blocks of 8 columns, for the tile's first mb x nb blocks.
 // SCALE: B's columns scaled by d[]; else B is lower triangular.
 template <bool SCALE>
-__device__ __forceinline__ void gemm_tile(double (&acc)[4][2][2], const double *A, const double *B, const double *d,
+__device__ __forceinline__ void gemm_tile(double (&acc)[2][2][2], const double *A, const double *B, const double *d,
                                           int kb, int mb, int nb, const TileBlocks &tb, int lane) {
     const bool two = tb.col(1) < nb;
-    if (tb.col(0) >= nb) return;
-    switch ((mb - tb.h + 1) >> 1) {  // the warp's rows in use
-        case 4: return gemm_rows<SCALE, 4>(acc, A, B, d, kb, two, tb, lane);
-        case 3: return gemm_rows<SCALE, 3>(acc, A, B, d, kb, two, tb, lane);
-        case 2: return gemm_rows<SCALE, 2>(acc, A, B, d, kb, two, tb, lane);
-        case 1: return gemm_rows<SCALE, 1>(acc, A, B, d, kb, two, tb, lane);
-    }
+    if (tb.col(0) >= nb || tb.row(0) >= mb) return;
+    if (tb.row(1) < mb) gemm_rows<SCALE, 2>(acc, A, B, d, kb, two, tb, lane);
+    else gemm_rows<SCALE, 1>(acc, A, B, d, kb, two, tb, lane);
 }
 
-// The 36 lower 8 x 8 blocks of a diagonal tile over 8 warps: rows 7 - p and p
-// (9 blocks) go to warps 2p (4 blocks) and 2p + 1 (5).
+// The 36 lower 8 x 8 blocks of a diagonal tile over 16 warps: the first to warp
+// 0, which starts the factorization with it, up to three neighbours of a row to
+// each of the others.
 struct DiagBlocks {
-    int p, e0;
-    __device__ __forceinline__ bool on(int i) const { return i < 4 || e0; }
-    __device__ __forceinline__ bool top(int i) const { return e0 + i < 8 - p; }
-    __device__ __forceinline__ int row(int i) const { return top(i) ? 7 - p : p; }
-    __device__ __forceinline__ int col(int i) const { return top(i) ? e0 + i : e0 + i - (8 - p); }
-    __device__ __forceinline__ int at(int i) const { return col(i) * 512 + row(i) * 64; }
+    int row, c0, n;
+    __device__ __forceinline__ int at(int i) const { return (c0 + i) * 512 + row * 64; }
 };
+__device__ __forceinline__ DiagBlocks diag_blocks(int warp) {
+    // hexadecimal digit w (from the right): warp w's row, first column, blocks
+    constexpr unsigned long long ROW = 0x0123344556667770ull, COL = 0x0002030305306300ull, NUM = 0x0232223332232331ull;
+    return DiagBlocks{(int)(ROW >> 4 * warp & 15), (int)(COL >> 4 * warp & 15), (int)(NUM >> 4 * warp & 15)};
+}
 template <int N>
-__device__ __forceinline__ void gemm_diag_n(double (&acc)[5][2], const double *A, const double *d, int kb,
+__device__ __forceinline__ void gemm_diag_n(double (&acc)[3][2], const double *A, const double *d, int kb,
                                             const DiagBlocks &db, int lane) {
-    const double *top = A + (7 - db.p) * 64, *low = A + db.p * 64;
+    double odd[N][2];
+#pragma unroll
+    for (int i = 0; i < N; i++) odd[i][0] = odd[i][1] = 0.0;
 #pragma unroll 2
     for (int k = 0; k < kb; k++) {
-        const double d0 = d[8 * k + (lane & 3)], d1 = d[8 * k + 4 + (lane & 3)];
-        double2 at = frag(top + k * 512, lane), al = frag(low + k * 512, lane), b[N];
-        at.x *= d0;
-        at.y *= d1;
-        al.x *= d0;
-        al.y *= d1;
+        double2 a = frag(A + k * 512 + db.row * 64, lane), b[N];
+        a.x *= d[8 * k + (lane & 3)];
+        a.y *= d[8 * k + 4 + (lane & 3)];
 #pragma unroll
-        for (int i = 0; i < N; i++) b[i] = frag(A + k * 512 + db.col(i) * 64, lane);
+        for (int i = 0; i < N; i++) b[i] = frag(A + k * 512 + (db.c0 + i) * 64, lane);
 #pragma unroll
-        for (int i = 0; i < N; i++) dmma(acc[i], db.top(i) ? at.x : al.x, b[i].x);
+        for (int i = 0; i < N; i++) {
+            dmma(acc[i], a.x, b[i].x);
+            dmma(odd[i], a.y, b[i].y);
+        }
+    }
 #pragma unroll
-        for (int i = 0; i < N; i++) dmma(acc[i], db.top(i) ? at.y : al.y, b[i].y);
+    for (int i = 0; i < N; i++) {
+        acc[i][0] += odd[i][0];
+        acc[i][1] += odd[i][1];
     }
 }
 // acc += A D A^T on the lower blocks, for the tile's first mb block rows.
-__device__ __forceinline__ void gemm_diag(double (&acc)[5][2], const double *A, const double *d, int kb, int mb,
+__device__ __forceinline__ void gemm_diag(double (&acc)[3][2], const double *A, const double *d, int kb, int mb,
                                           const DiagBlocks &db, int lane) {
-    if (db.e0) {
-        if (db.p < mb) gemm_diag_n<5>(acc, A, d, kb, db, lane);
-    } else if (7 - db.p < mb) {
-        gemm_diag_n<4>(acc, A, d, kb, db, lane);
-    }
+    if (db.row >= mb) return;
+    if (db.n == 3) gemm_diag_n<3>(acc, A, d, kb, db, lane);
+    else if (db.n == 2) gemm_diag_n<2>(acc, A, d, kb, db, lane);
+    else if (db.n == 1) gemm_diag_n<1>(acc, A, d, kb, db, lane);
 }
 
 // Row block w of A times v (first kb blocks of 8 columns): lane's partial sum
 // for row 8w + lane / 4.
 __device__ __forceinline__ double row_dot(const double *A, const double *v, int kb, int w, int lane) {
     double s0 = 0.0, s1 = 0.0;
-#pragma unroll 4
+#pragma unroll 2
     for (int k = 0; k < kb; k++) {
         const double2 a = frag(A + k * 512 + w * 64, lane);
         s0 = fma(a.x, v[8 * k + (lane & 3)], s0);
@@ -336,7 +344,8 @@ __device__ __forceinline__ double reciprocal(double d) {
 // its L: lane 4r + q holds columns q and q + 4 of row r, of the whole symmetric
 // block, so a pivot row is at hand in its own lanes' registers.  Two pivots a
 // step through the inverse of their 2 x 2 block P = [p g; g c], so the chain
-// holds one reciprocal per two pivots: row r's multipliers are (a_rk, a_r,k+1) P^-1.
+// holds one reciprocal per two pivots: row r's multipliers are (a_rk, a_r,k+1)
+// P^-1.  What turns the blocks into single pivots comes after the last pair.
 __device__ __forceinline__ void factor8(Smem &sm, int s, int lane, unsigned long long *flags) {
     const unsigned FULL = 0xffffffffu;
     const int r = lane >> 2, q = lane & 3;
@@ -348,22 +357,24 @@ __device__ __forceinline__ void factor8(Smem &sm, int s, int lane, unsigned long
         a[i] = blk[nd_at(max(r, c), min(r, c))];
         m[i] = c == r ? 1.0 : 0.0;
     }
-    double dr = 1.0;
+    double pr = 1.0, gr = 0.0, cr = 1.0;  // the 2 x 2 block of this row's pair
 #pragma unroll
     for (int k = 0; k < 8; k += 2) {
         const int i = k >> 2, q0 = k & 3;
         const double p = __shfl_sync(FULL, a[i], 4 * k + q0);
         const double g = __shfl_sync(FULL, a[i], 4 * k + 4 + q0);
         const double c = __shfl_sync(FULL, a[i], 4 * k + 4 + q0 + 1);
+        if ((r & 6) == k) {
+            pr = p;
+            gr = g;
+            cr = c;
+        }
+        if (k == 6) break;  // the last rows are done
         const double u = __shfl_sync(FULL, a[i], (lane & ~3) | q0);
         const double v = __shfl_sync(FULL, a[i], (lane & ~3) | (q0 + 1));
-        const double det = fma(p, c, -(g * g));
-        const double rd = reciprocal(det), rp = reciprocal(p);
-        const double l = g * rp;  // L_k+1,k
-        if (r == k) dr = p;
-        if (r == k + 1) dr = fma(-l, g, c);
-        double w0 = -fma(c, u, -(g * v)) * rd, w1 = -fma(p, v, -(g * u)) * rd;
-        if (r <= k + 1) w0 = w1 = 0.0;
+        double rd = reciprocal(fma(p, c, -(g * g)));
+        if (r <= k + 1) rd = 0.0;
+        const double w0 = fma(g, v, -(c * u)) * rd, w1 = fma(g, u, -(p * v)) * rd;
 #pragma unroll
         for (int j = 0; j < 2; j++) {
             if (4 * j + 3 > k + 1) {  // some lane's column is past the pivots
@@ -373,8 +384,18 @@ __device__ __forceinline__ void factor8(Smem &sm, int s, int lane, unsigned long
             if (4 * j <= k + 1) {
                 const double x0 = __shfl_sync(FULL, m[j], 4 * k + q), x1 = __shfl_sync(FULL, m[j], 4 * k + 4 + q);
                 m[j] = fma(w1, x1, fma(w0, x0, m[j]));
-                if (r == k + 1) m[j] = fma(-l, x0, m[j]);
             }
+        }
+    }
+    // within each pair: L_k+1,k = g / p, the second pivot c - g^2 / p
+    const double l = gr * reciprocal(pr);
+    double dr = pr;
+    {
+        const double m0 = __shfl_sync(FULL, m[0], lane & ~4), m1 = __shfl_sync(FULL, m[1], lane & ~4);
+        if (r & 1) {
+            dr = fma(-l, gr, cr);
+            m[0] = fma(-l, m0, m[0]);
+            m[1] = fma(-l, m1, m[1]);
         }
     }
     // a pivot that the reciprocals could not take makes itself or a later one fail this
@@ -405,7 +426,7 @@ __device__ __forceinline__ void panel_block(Smem &sm, int s, int rb, int lane) {
     store_block(p, w, lane);
 }
 
-// Blocks u0, u0 + 7, ... (N of them, below `count`) of the lower triangle that
+// Blocks u0, u0 + 15, ... (N of them, below `count`) of the lower triangle that
 // starts at block `first` -= L D L^T of block column s; a block's number is
 // its row's first, i (i + 1) / 2, plus its column.  All loads before the products.
 template <int N>
@@ -416,7 +437,7 @@ __device__ __forceinline__ void trail_blocks(Smem &sm, int s, int first, int u0,
     const double d0 = -sm.d[8 * s + (lane & 3)], d1 = -sm.d[8 * s + 4 + (lane & 3)];
 #pragma unroll
     for (int n = 0; n < N; n++) {
-        const int u = u0 + 7 * n < count ? u0 + 7 * n : 0;
+        const int u = u0 + 15 * n < count ? u0 + 15 * n : 0;
         const int i = (u >= 1) + (u >= 3) + (u >= 6) + (u >= 10) + (u >= 15) + (u >= 21), o = u - i * (i + 1) / 2;
         at[n] = (first + o) * 512 + (first + i) * 64;
         x[n] = frag(sm.c + s * 512 + (first + i) * 64, lane);
@@ -434,29 +455,38 @@ __device__ __forceinline__ void trail_blocks(Smem &sm, int s, int first, int u0,
         acc[n][0] += acc2[n][0];
         acc[n][1] += acc2[n][1];
         const double2 v = to_stored(acc[n], lane);
-        if (u0 + 7 * n < count) *reinterpret_cast<double2 *>(sm.c + at[n] + 2 * stored_lane(lane)) = v;
+        if (u0 + 15 * n < count) *reinterpret_cast<double2 *>(sm.c + at[n] + 2 * stored_lane(lane)) = v;
     }
 }
 
-// L D L^T of the 64 x 64 block in sm.c (lower part), warps 0-7: its inverse
+// L D L^T of the 64 x 64 block in sm.c (lower part), warps 0-15: its inverse
 // (sm.inv, and in global memory at g), sm.d, sm.dinv, and z = L^-1 r (at gz; D and
-// 1/D beside it).  Eight columns a step.  Warp 0 runs the chain: it factors the
-// 8 x 8 block, then forms the L rows and updates the block that the next step
-// factors, while the other warps do the step's remaining rows and blocks and
-// the inverse's next block row.  Latency-bound: a step is a chain of about 25
-// dependent FP64 operations, ten shuffles and two barriers.
-__device__ void factor64(Smem &sm, int warp, int lane, double *g, double *gz, unsigned long long *flags) {
+// 1/D beside it; `release` is arrived at after the first step).  Eight columns a
+// step.  Warp 0 runs the chain: it factors the 8 x 8 block, then forms the L rows
+// and updates the block that the next step factors, while the other warps do the
+// step's remaining rows and blocks and the inverse's next block row.  Latency-
+// bound, 2,000 clocks a step: the 8 x 8 block 1,150, the L rows 190, the update
+// 190, the rest barriers and the other warps' products (8 warps: 2,500 clocks).
+__device__ void factor64(Smem &sm, int warp, int lane, double *g, double *gz, unsigned long long *release,
+                         unsigned long long *flags) {
+    auto z_rows = [&](int w) {
+        const double zr = sum_quad(row_dot(sm.inv, sm.r, 8, w, lane));
+        if ((lane & 3) == 0) gz[8 * w + (lane >> 2)] = zr;
+    };
+#pragma unroll 1
     for (int s = 0; s < 8; s++) {
         if (warp == 0) {
             factor8(sm, s, lane, flags);
         } else if (s > 0) {
             // the rest of step s - 1's update, then tt = (L_s,0..s-1 Linv_0..s-1)^T
             const int n = 8 - s, count = n * (n + 1) / 2;  // block 0 is warp 0's
-            if (s < 4) trail_blocks<4>(sm, s - 1, s, warp, count, lane);
-            else if (s < 7) trail_blocks<2>(sm, s - 1, s, warp, count, lane);
-            if (warp <= s) {
-                const int cb = warp - 1;
+            if (count > 16) trail_blocks<2>(sm, s - 1, s, warp, count, lane);
+            else if (warp < count) trail_blocks<1>(sm, s - 1, s, warp, count, lane);
+            if (warp == 8) z_rows(s - 1);  // which has no part in the next
+            if (15 - warp < s) {
+                const int cb = 15 - warp;
                 double acc[2] = {0.0, 0.0}, acc2[2] = {0.0, 0.0};
+#pragma unroll 1
                 for (int k = cb; k < s; k++) {
                     const double2 x = frag(sm.c + k * 512 + s * 64, lane);
                     const double2 y = frag(sm.invt + k * 448 + cb * 64, lane);
@@ -466,12 +496,9 @@ __device__ void factor64(Smem &sm, int warp, int lane, double *g, double *gz, un
 #pragma unroll
                 for (int e = 0; e < 2; e++) sm.tt[at56(8 * cb + 2 * (lane & 3) + e, lane >> 2)] = acc[e] + acc2[e];
             }
-            if (warp == 7) {
-                const double zr = sum_quad(row_dot(sm.inv, sm.r, 8, s - 1, lane));
-                if ((lane & 3) == 0) gz[8 * (s - 1) + (lane >> 2)] = zr;
-            }
         }
         sync_work();
+        if (s == 0 && release && lane == 0) bar_arrive(release);
         if (warp == 0 && s < 7) {
             panel_block(sm, s, s + 1, lane);
             asm volatile("barrier.cta.arrive 3, %0;" ::"n"(WORK) : "memory");
@@ -484,7 +511,7 @@ __device__ void factor64(Smem &sm, int warp, int lane, double *g, double *gz, un
         // the inverse's block row s: -Linv8 (L_s Linv)
         if (warp == 1)
             *reinterpret_cast<double2 *>(g + s * 512 + s * 64 + 2 * lane) = frag(sm.inv + s * 512 + s * 64, lane);
-        for (int cb = 7 - warp; cb < s && (warp > 0 || s == 7); cb += 7) {
+        if (const int cb = 15 - warp; cb < s) {
             double acc[2] = {0.0, 0.0}, acc2[2] = {0.0, 0.0};
             const double2 x = frag(sm.inv + s * 512 + s * 64, lane), y = frag(sm.tt + cb * 64, lane);
             dmma(acc, -x.x, y.x);
@@ -493,6 +520,10 @@ __device__ void factor64(Smem &sm, int warp, int lane, double *g, double *gz, un
             acc[1] += acc2[1];
             store_block(sm.inv + cb * 512 + s * 64, acc, lane);
             store_block(g + cb * 512 + s * 64, acc, lane);
+            if (s == 7) {
+                const double v = sum_quad(fma(acc[0], sm.r[8 * cb + 2 * (lane & 3)], acc[1] * sm.r[8 * cb + 2 * (lane & 3) + 1]));
+                if ((lane & 3) == 0) sm.z7[cb][lane >> 2] = v;
+            }
             if (s < 7) {
 #pragma unroll
                 for (int e = 0; e < 2; e++) sm.invt[at56(8 * cb + 2 * (lane & 3) + e, 8 * s + (lane >> 2))] = acc[e];
@@ -500,10 +531,19 @@ __device__ void factor64(Smem &sm, int warp, int lane, double *g, double *gz, un
         }
         if (s < 7) asm volatile("barrier.cta.sync 3, %0;" ::"n"(WORK) : "memory");
     }
+    if (warp == 0) {
+        const double2 x = frag(sm.inv + 7 * 512 + 7 * 64, lane);
+        const double v = sum_quad(fma(x.x, sm.r[56 + (lane & 3)], x.y * sm.r[60 + (lane & 3)]));
+        if ((lane & 3) == 0) sm.z7[7][lane >> 2] = v;
+    }
     sync_work();
     if (warp == 0) {
-        const double zr = sum_quad(row_dot(sm.inv, sm.r, 8, 7, lane));
-        if ((lane & 3) == 0) gz[56 + (lane >> 2)] = zr;
+        if (lane < 8) {
+            double v = 0.0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) v += sm.z7[k][lane];
+            gz[56 + lane] = v;
+        }
     } else if (warp < 5) {
         const int i = 32 * (warp - 1) + lane;
         gz[T + i] = i < T ? sm.d[i] : sm.dinv[i - T];
@@ -592,8 +632,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_nd_factor(NdArgs a) {
 
     TileBlocks tb;
     tb.h = warp >> 2;
-    tb.c0 = tb.h ? 3 - (warp & 3) : warp & 3;
-    const DiagBlocks db{warp >> 1, (warp & 1) * 4};
+    tb.c0 = tb.h & 1 ? 3 - (warp & 3) : warp & 3;
+    const DiagBlocks db = diag_blocks(warp);
+    const int rw = warp - 8;           // warps 8-15: the row block of the right-hand side they sum
     unsigned pubs = 0;
     // hands tiles p and q (-1: none) to the publisher; every work warp calls it after its writes
     auto publish = [&](int p, int q) {
@@ -607,7 +648,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_nd_factor(NdArgs a) {
         if (lane == 0) bar_arrive(&sm.pub_full[s]);
         pubs++;
     };
-    double accx[4][2][2], accd[5][2], rs = 0.0;
+    double accx[2][2][2], accd[3][2], rs = 0.0;
     for (unsigned it = 0;; it++) {
         const int s = it % STAGES;
         if (!all_work(bar_wait(&sm.full[s], (it / STAGES) & 1, &sm.abort))) {
@@ -624,23 +665,27 @@ __global__ void __launch_bounds__(THREADS, 1) k_nd_factor(NdArgs a) {
         const double *A = sm.stage[s][0], *B = sm.stage[s][1], *z = sm.zd[s], *D = z + T, *Di = z + 2 * T;
         if (im.b == ND_BEGIN) {
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < 2; i++)
 #pragma unroll
                 for (int j = 0; j < 2; j++) accx[i][j][0] = accx[i][j][1] = 0.0;
 #pragma unroll
-            for (int i = 0; i < 5; i++) accd[i][0] = accd[i][1] = 0.0;
+            for (int i = 0; i < 3; i++) accd[i][0] = accd[i][1] = 0.0;
             rs = 0.0;
             if (!partial) {
-                // J's entries, now: the loads would be on the chain later.  sm.c takes the
-                // off-diagonal tile, sm.inv (free until the factor) the diagonal one.
+                // J's entries, now: the loads would be on the chain later.  They go through sm.c
+                // (the off-diagonal tile) and sm.inv (the diagonal one) into the sums.
                 const int x0 = diag ? task.xent0 : task.ent0, x1 = diag ? task.xent1 : task.ent1;
+                const bool entries = x1 > x0;
+#pragma unroll 1
                 for (int i = t; i < TT / 2; i += WORK) {
-                    if (x1 > x0) reinterpret_cast<double2 *>(sm.c)[i] = make_double2(0.0, 0.0);
+                    if (entries) reinterpret_cast<double2 *>(sm.c)[i] = make_double2(0.0, 0.0);
                     if (diag) reinterpret_cast<double2 *>(sm.inv)[i] = make_double2(0.0, 0.0);
                 }
-                sync_work();
+                if (entries || diag) sync_work();
+#pragma unroll 1
                 for (int e = x0 + t; e < x1; e += WORK) sm.c[a.ent_at[e]] = a.kval[a.ent_src[e]];
                 if (diag) {
+#pragma unroll 1
                     for (int e = task.ent0 + t; e < task.ent1; e += WORK) sm.inv[a.ent_at[e]] = a.kval[a.ent_src[e]];
                     sync_work();
                     if (t < T) {
@@ -649,21 +694,41 @@ __global__ void __launch_bounds__(THREADS, 1) k_nd_factor(NdArgs a) {
                         sm.r[t] = u >= 0 ? a.b[u] : 0.0;
                     }
                 }
+                if (entries || diag) sync_work();
+                if (entries) {
+#pragma unroll
+                    for (int i = 0; i < 2; i++)
+#pragma unroll
+                        for (int j = 0; j < 2; j++) {
+                            load_block(sm.c + tb.at(i, j), accx[i][j], lane);
+                            accx[i][j][0] = -accx[i][j][0];
+                            accx[i][j][1] = -accx[i][j][1];
+                        }
+                }
+                if (diag) {
+#pragma unroll
+                    for (int i = 0; i < 3; i++)
+                        if (i < db.n) {
+                            load_block(sm.inv + db.at(i), accd[i], lane);
+                            accd[i][0] = -accd[i][0];
+                            accd[i][1] = -accd[i][1];
+                        }
+                }
             }
         } else if (im.b == ND_ADD || im.b == ND_ADDX) {
             if (diag && im.b == ND_ADD) {
 #pragma unroll
-                for (int i = 0; i < 5; i++)
-                    if (db.on(i)) {
+                for (int i = 0; i < 3; i++)
+                    if (i < db.n) {
                         double v[2];
                         load_block(A + db.at(i), v, lane);
                         accd[i][0] += v[0];
                         accd[i][1] += v[1];
                     }
-                if ((lane & 3) == 0) rs += z[8 * warp + (lane >> 2)];
+                if (rw >= 0 && (lane & 3) == 0) rs += z[8 * rw + (lane >> 2)];
             } else {
 #pragma unroll
-                for (int i = 0; i < 4; i++)
+                for (int i = 0; i < 2; i++)
 #pragma unroll
                     for (int j = 0; j < 2; j++) {
                         double v[2];
@@ -676,63 +741,69 @@ __global__ void __launch_bounds__(THREADS, 1) k_nd_factor(NdArgs a) {
             if (im.b >= 0) gemm_tile<true>(accx, A, B, D, im.kblocks, diag ? nb : mb, diag ? pb : nb, tb, lane);
             if (diag) {
                 gemm_diag(accd, A, D, im.kblocks, nb, db, lane);
-                rs += row_dot(A, z, im.kblocks, warp, lane);
+                if (rw >= 0) rs += row_dot(A, z, im.kblocks, rw, lane);
             }
         } else {
             // the tile so far, C = K - products, then L = C Linv^T D^-1
-            const bool entries = diag ? task.xent1 > task.xent0 : task.ent1 > task.ent0;
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < 2; i++)
 #pragma unroll
                 for (int j = 0; j < 2; j++) {
-                    double *p = sm.c + tb.at(i, j), v[2] = {0.0, 0.0};
-                    if (entries) load_block(p, v, lane);
-                    v[0] -= accx[i][j][0];
-                    v[1] -= accx[i][j][1];
-                    __syncwarp();
-                    store_block(p, v, lane);
+                    const double v[2] = {-accx[i][j][0], -accx[i][j][1]};
+                    store_block(sm.c + tb.at(i, j), v, lane);
                     accx[i][j][0] = accx[i][j][1] = 0.0;
                 }
             sync_work();
             gemm_tile<false>(accx, sm.c, A, nullptr, im.kblocks, diag ? nb : mb, im.kblocks, tb, lane);
-            if (diag) sync_work();  // the tile is read by all before it is overwritten
             const int to = diag ? xout : out;
-            double *g = a.tile + (size_t)to * TT;
+            double *g = a.tile + (size_t)to * TT, *l = sm.stage[s][1];  // (no second operand came)
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < 2; i++)
 #pragma unroll
                 for (int j = 0; j < 2; j++) {
                     const int cb = tb.col(j);
                     accx[i][j][0] *= Di[8 * cb + 2 * (lane & 3)];
                     accx[i][j][1] *= Di[8 * cb + 2 * (lane & 3) + 1];
+                    if (diag) store_block(l + tb.at(i, j), accx[i][j], lane);
                     store_block(g + tb.at(i, j), accx[i][j], lane);
-                    if (diag) store_block(sm.c + tb.at(i, j), accx[i][j], lane);
                 }
-            if (diag) {
-                sync_work();
-                gemm_diag(accd, sm.c, D, im.kblocks, nb, db, lane);
-                rs += row_dot(sm.c, z, im.kblocks, warp, lane);
-            }
             publish(to, -1);
+            if (diag) {
+                // the last products of the diagonal block; warp 0 has the first block's only and goes
+                // on to factor it while the others finish theirs
+                sync_work();
+                gemm_diag(accd, l, D, im.kblocks, nb, db, lane);
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+                    if (i < db.n) {
+                        const double v[2] = {-accd[i][0], -accd[i][1]};
+                        store_block(sm.c + db.at(i), v, lane);
+                    }
+                if (rw >= 0) {
+                    rs = sum_quad(rs + row_dot(l, z, im.kblocks, rw, lane));
+                    if ((lane & 3) == 0) sm.r[8 * rw + (lane >> 2)] -= rs;
+                }
+            }
         }
         __syncwarp();
-        if (lane == 0) bar_arrive(&sm.empty[s]);
+        const bool fused = diag && im.b == ND_INV;  // the stage is still read: factor64 releases it
+        if (!fused && lane == 0) bar_arrive(&sm.empty[s]);
         if (!last) continue;
         if (partial) {
             // the sums as they are
             if (diag) {
                 double *g = a.tile + (size_t)out * TT;
 #pragma unroll
-                for (int i = 0; i < 5; i++)
-                    if (db.on(i)) store_block(g + db.at(i), accd[i], lane);
+                for (int i = 0; i < 3; i++)
+                    if (i < db.n) store_block(g + db.at(i), accd[i], lane);
                 rs = sum_quad(rs);
-                if ((lane & 3) == 0) a.zd[(size_t)(a.ncol + out - a.ntile) * ZD + 8 * warp + (lane >> 2)] = rs;
+                if (rw >= 0 && (lane & 3) == 0) a.zd[(size_t)(a.ncol + out - a.ntile) * ZD + 8 * rw + (lane >> 2)] = rs;
             }
             const int to = diag ? xout : out;
             if (to >= 0) {
                 double *g = a.tile + (size_t)to * TT;
 #pragma unroll
-                for (int i = 0; i < 4; i++)
+                for (int i = 0; i < 2; i++)
 #pragma unroll
                     for (int j = 0; j < 2; j++) store_block(g + tb.at(i, j), accx[i][j], lane);
             }
@@ -740,22 +811,20 @@ __global__ void __launch_bounds__(THREADS, 1) k_nd_factor(NdArgs a) {
             continue;
         }
         if (!diag) continue;
-        // the diagonal block: C = J - products, factor, inverse, z = Linv (b - products)
-        sync_work();
+        // the diagonal block: factor, inverse, z = Linv (b - products)
+        if (!fused) {
 #pragma unroll
-        for (int i = 0; i < 5; i++)
-            if (db.on(i)) {
-                const int o = db.at(i);
-                double v[2];
-                load_block(sm.inv + o, v, lane);
-                v[0] -= accd[i][0];
-                v[1] -= accd[i][1];
-                store_block(sm.c + o, v, lane);
-            }
-        rs = sum_quad(rs);
-        if ((lane & 3) == 0) sm.r[8 * warp + (lane >> 2)] -= rs;
-        sync_work();
-        factor64(sm, warp, lane, a.tile + (size_t)out * TT, a.zd + (size_t)J * ZD, a.flags);
+            for (int i = 0; i < 3; i++)
+                if (i < db.n) {
+                    const double v[2] = {-accd[i][0], -accd[i][1]};
+                    store_block(sm.c + db.at(i), v, lane);
+                }
+            rs = sum_quad(rs);
+            if (rw >= 0 && (lane & 3) == 0) sm.r[8 * rw + (lane >> 2)] -= rs;
+            sync_work();
+        }
+        factor64(sm, warp, lane, a.tile + (size_t)out * TT, a.zd + (size_t)J * ZD, fused ? &sm.empty[s] : nullptr,
+                 a.flags);
         publish(out, -1);
     }
 }
@@ -763,7 +832,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_nd_factor(NdArgs a) {
 // ---- triangular solves with the stored factor ------------------------------------------
 
 constexpr int SOLVE_STAGES = 6;
-constexpr int SOLVE_THREADS = WORK + 32;  // and the producer's warp
+constexpr int SOLVE_WORK = 256;           // threads of warps 0-7
+constexpr int SOLVE_THREADS = SOLVE_WORK + 32;  // and the producer's warp
 
 struct SolveArgs {
     const int *ptr, *tiles;            // per column: the tiles it takes, in order (null tiles: tile ids ptr + 1 ..)
@@ -800,13 +870,13 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
     if (t == 0) {
         for (int s = 0; s < SOLVE_STAGES; s++) {
             bar_init(&sm.full[s], 1);
-            bar_init(&sm.empty[s], WORK / 32);
+            bar_init(&sm.empty[s], SOLVE_WORK / 32);
         }
         sm.abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (warp == WORK / 32) {
+    if (warp == SOLVE_WORK / 32) {
         if (lane) return;
         unsigned it = 0;
         bool ok = true;
@@ -880,7 +950,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
             if (ok) continue;
             sm.abort = 1;
         }
-        if (!all_work(ok)) {
+        if (!all_work<SOLVE_WORK>(ok)) {
             if (t == 0) give_up(a.ctl + 1, a.flags);
             return;
         }
@@ -905,7 +975,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
                 sm.v[r] = u >= 0 ? a.b[u] - s0 : 0.0;
             }
         }
-        sync_work();
+        sync_work<SOLVE_WORK>();
         if (BACK) {
             s0 = s1 = 0.0;
 #pragma unroll
@@ -934,7 +1004,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
             if ((lane & 3) == 0) a.zd[(size_t)J * ZD + 8 * warp + (lane >> 2)] = zr;
         }
         s0 = s1 = 0.0;
-        sync_work();
+        sync_work<SOLVE_WORK>();
         if (t == 0) st_release(a.flag + J, a.epoch);
         if (lane == 0) bar_arrive(&sm.empty[s]);
     }
