@@ -66,7 +66,7 @@ enum {
 
 /* FESolver::Method, src/FESolver.h:26, and two sparse methods of this library:
  * SPARSE_CG is the Lapack method's single Newton step (src/FESolver.cpp:301-317)
- * with J y = G solved by Jacobi-preconditioned conjugate gradients in FP64 on
+ * with J y = G solved by preconditioned conjugate gradients in FP64 on
  * the sparse K (||G - J y|| <= rtol ||G||, mp_set_sparse_solver);
  * SPARSE_NEWTON is the NonLinear method's loop (src/FESolver.cpp:324-364: F1
  * accumulating, up to 10 iterations, stop at ||y||/neq < 1e-2) with the same

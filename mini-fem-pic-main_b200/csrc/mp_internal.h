@@ -200,7 +200,9 @@ struct mp_ctx {
     int *sp_col = nullptr;                // [sp_slots]
     double *sp_val = nullptr;             // [sp_slots]
     long long sp_nnz = 0, sp_slots = 0;
+    unsigned sp_changes = 0;              // counts the times sp_val was written
     void *sparse_scratch = nullptr;       // conjugate-gradient work (mp_sparse.cu)
+    void *cg_levels = nullptr;            // multilevel conjugate gradients' plan (mp_cg_levels.cu)
     double cg_rtol = 1e-12;               // ||G - J y|| <= cg_rtol ||G||
     int cg_max_it = 20000;
     int gs_max_sweeps = 10000;            // solveLinear's sweep limit (src/FESolver.cpp:575)
@@ -305,7 +307,12 @@ int fe_sparse_from_host(mp_ctx *ctx, const double *const *rows, const double *de
 int fe_residual_sparse(mp_ctx *ctx);
 int fe_resid_j_sparse(mp_ctx *ctx, const double *y, const double *b, double *r, float *r32, double *sums);
 int fe_solve_cg(mp_ctx *ctx, mp_newton_stats *st);
-int cg_enqueue(mp_ctx *ctx, const unsigned **stop);
+int cg_enqueue(mp_ctx *ctx, const unsigned **stop, bool diagonal = false);
+bool cg_again(mp_ctx *ctx);
+int cg_levels_setup(mp_ctx *ctx, const std::vector<long long> &rowp, const std::vector<int> &cols,
+                    const std::vector<long long> &slot);
+int cg_levels_enqueue(mp_ctx *ctx, unsigned *sync, double *out, bool *done);
+void cg_levels_free(mp_ctx *ctx);
 int cg_finish(mp_ctx *ctx, mp_newton_stats *st);
 int fe_step_lean(mp_ctx *ctx, const double *den, int method, int form, bool first, mp_newton_stats *st, double *l2);
 void solve_free(mp_ctx *ctx);

@@ -225,6 +225,13 @@ int fe_step_lean(mp_ctx *ctx, const double *den, int method, int form, bool firs
     MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     NewtonState s;
     newton_read(ctx, &s);
+    if (cg && cg_again(ctx)) {
+        if ((rc = cg_enqueue(ctx, &stop, true))) return rc;
+        MP_CUDA(ctx, cudaMemsetAsync(ctx->scal, 0, sizeof(double), ctx->stream));
+        if ((rc = newton_update(ctx, stop))) return rc;
+        MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        newton_read(ctx, &s);
+    }
     if (cg || gs) {
         if ((rc = cg ? cg_finish(ctx, st) : gs_finish(ctx, st))) return rc;
         *l2 = s.l2;

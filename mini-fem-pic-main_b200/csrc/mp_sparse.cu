@@ -1,7 +1,9 @@
 // Sparse field solve: K in sliced-ELLPACK form (SELL-32), assembled on the
 // device; G = K d - F0 - F1 by a sparse product in the reference's column
-// order; J y = G (J = K - diag(FP)) by Jacobi-preconditioned conjugate
-// gradients in FP64, one cooperative kernel per solve.
+// order; J y = G (J = K - diag(FP)) by conjugate gradients in FP64, one
+// cooperative kernel per solve: the multilevel form of mp_cg_levels.cu, and here
+// the form preconditioned by J's diagonal, which takes meshes outside the other's
+// range and decides what that one could not solve.
 //
 // K has about 15 nonzeros per row (the 14 mesh neighbours of a node and the
 // node itself), so the dense neq x neq storage of FESolver (src/FESolver.cpp:
@@ -431,6 +433,7 @@ struct SparseScratch {
     double *out_host = nullptr;  // pinned [4] + status
     long long vec_len = 0;
     int part_len = 0;
+    bool levels = false;         // the solve under way is the multilevel one
 };
 
 SparseScratch *scratch_of(mp_ctx *ctx) {
@@ -449,6 +452,7 @@ void sparse_free(mp_ctx *ctx) {
     ctx->sp_col = nullptr;
     ctx->sp_val = nullptr;
     ctx->sp_nnz = ctx->sp_slots = 0;
+    cg_levels_free(ctx);
     if (ctx->sparse_scratch) {
         SparseScratch *s = static_cast<SparseScratch *>(ctx->sparse_scratch);
         void *d2[] = {s->vec, s->part, s->sync, s->out};
@@ -515,18 +519,18 @@ int sparse_setup(mp_ctx *ctx, const std::vector<int> &LM, const std::vector<int>
     ctx->csr_ptr.clear();
     ctx->csr_col.clear();
     ctx->csr_slot.clear();
-    if (ctx->fe_storage == MP_FE_STORAGE_DENSE) {
-        ctx->csr_slot.resize(nnz);
-        for (int P = 0; P < neq; P++)
-            for (long long k = rowp[P]; k < rowp[P + 1]; k++)
-                ctx->csr_slot[k] = ptr[P >> 5] + 32ll * (k - rowp[P]) + (P & 31);
-        ctx->csr_ptr = std::move(rowp);
-        ctx->csr_col = std::move(cols);
-    }
+    std::vector<long long> slot(nnz);
+    for (int P = 0; P < neq; P++)
+        for (long long k = rowp[P]; k < rowp[P + 1]; k++) slot[k] = ptr[P >> 5] + 32ll * (k - rowp[P]) + (P & 31);
+    if (ctx->fe_storage == MP_FE_STORAGE_SPARSE) return cg_levels_setup(ctx, rowp, cols, slot);
+    ctx->csr_slot = std::move(slot);  // the plans of the dense storage's solvers are made when first needed
+    ctx->csr_ptr = std::move(rowp);
+    ctx->csr_col = std::move(cols);
     return MP_OK;
 }
 
 int fe_assemble_sparse(mp_ctx *ctx) {
+    ctx->sp_changes++;
     MP_CUDA(ctx, cudaMemsetAsync(ctx->sp_val, 0, sizeof(double) * std::max(1ll, ctx->sp_slots), ctx->stream));
     MP_CUDA(ctx, cudaMemsetAsync(ctx->scal + 4, 0, sizeof(double), ctx->stream));
     unsigned *bad = reinterpret_cast<unsigned *>(ctx->scal + 4);
@@ -544,6 +548,7 @@ int fe_assemble_sparse(mp_ctx *ctx) {
 }
 
 int fe_sparse_from_dense(mp_ctx *ctx) {
+    ctx->sp_changes++;
     const long long ld = (ctx->neq + 31) & ~31ll;
     int th = 128;
     k_dense_to_sell<<<(ctx->neq + th - 1) / th, th, 0, ctx->stream>>>(ctx->neq, ld, ctx->K, ctx->sp_len, ctx->sp_ptr,
@@ -605,6 +610,7 @@ int fe_pattern_fits(mp_ctx *ctx, bool *fits) {
 
 // K given on the host, sparse storage only: gather the nonzeros on the host.
 int fe_sparse_from_host(mp_ctx *ctx, const double *const *rows, const double *dense) {
+    ctx->sp_changes++;
     const int neq = ctx->neq;
     const int slices = (neq + 31) / 32;
     std::vector<int> len(neq);
@@ -689,10 +695,8 @@ cudaError_t launch_cg(const CgArgs &a, int nb, cudaStream_t stream) {
 // Rows are split in contiguous runs of rows_per_block (>= CG_THREADS) over at
 // most one block per SM; a thread keeps its rows' state in registers up to 4
 // rows (n <= 4 * 512 * SMs), in global memory beyond.
-// *stop: a device word that is not zero when the solve failed.
-int cg_enqueue(mp_ctx *ctx, const unsigned **stop) {
+static int cg_diagonal(mp_ctx *ctx, SparseScratch *s) {
     const int n = ctx->neq;
-    SparseScratch *s = scratch_of(ctx);
     // one row a thread while the rows fit one block per SM: a thread's rows are
     // worked one after the other, which costs more than the longer grid-wide
     // rounds of more blocks (measured: 7.1 us an iteration at 8,379 unknowns
@@ -715,12 +719,6 @@ int cg_enqueue(mp_ctx *ctx, const unsigned **stop) {
         MP_CUDA(ctx, cudaMalloc(&s->part, sizeof(double) * 6 * nb));
         s->part_len = 6 * nb;
     }
-    if (!s->sync) {
-        MP_CUDA(ctx, cudaMalloc(&s->sync, sizeof(unsigned) * 4));
-        MP_CUDA(ctx, cudaMalloc(&s->out, sizeof(double) * 4));
-        MP_CUDA(ctx, cudaHostAlloc(&s->out_host, sizeof(double) * 6, 0));
-    }
-    MP_CUDA(ctx, cudaMemsetAsync(s->sync, 0, sizeof(unsigned) * 4, ctx->stream));
     MP_CUDA(ctx, cudaMemsetAsync(s->part, 0xFF, sizeof(double) * 6 * nb, ctx->stream));  // every slot EMPTY
     CgArgs a;
     a.n = n;
@@ -748,10 +746,38 @@ int cg_enqueue(mp_ctx *ctx, const unsigned **stop) {
                                            : launch_cg<0>(a, nb, ctx->stream);
     MP_CUDA(ctx, e);
     ++ctx->launches;
+    return MP_OK;
+}
+
+// The same by the multilevel preconditioner where that applies, else (or with
+// `diagonal`) by J's diagonal.  *stop: a device word that is not zero when the
+// solve failed.
+int cg_enqueue(mp_ctx *ctx, const unsigned **stop, bool diagonal) {
+    SparseScratch *s = scratch_of(ctx);
+    if (!s->sync) {
+        MP_CUDA(ctx, cudaMalloc(&s->sync, sizeof(unsigned) * 4));
+        MP_CUDA(ctx, cudaMalloc(&s->out, sizeof(double) * 4));
+        MP_CUDA(ctx, cudaHostAlloc(&s->out_host, sizeof(double) * 6, 0));
+    }
+    MP_CUDA(ctx, cudaMemsetAsync(s->sync, 0, sizeof(unsigned) * 4, ctx->stream));
+    int rc;
+    s->levels = false;
+    if (!diagonal && (rc = cg_levels_enqueue(ctx, s->sync, s->out, &s->levels))) return rc;
+    if (!s->levels && (rc = cg_diagonal(ctx, s))) return rc;
     MP_CUDA(ctx, cudaMemcpyAsync(s->out_host, s->out, sizeof(double) * 4, cudaMemcpyDeviceToHost, ctx->stream));
     MP_CUDA(ctx, cudaMemcpyAsync(s->out_host + 4, s->sync + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     if (stop) *stop = s->sync + 1;
     return MP_OK;
+}
+
+// Whether the solve that was waited for is to be done again with J's diagonal
+// alone: the multilevel form has ended without a solution, which the plain
+// iteration decides then (an indefinite J, the iteration limit).
+bool cg_again(mp_ctx *ctx) {
+    const SparseScratch *s = scratch_of(ctx);
+    unsigned status;
+    std::memcpy(&status, s->out_host + 4, sizeof(unsigned));
+    return s->levels && status && !(status & CG_TIMEOUT);
 }
 
 // The solve's results, after the stream has been waited for.
@@ -777,6 +803,10 @@ int fe_solve_cg(mp_ctx *ctx, mp_newton_stats *st) {
     int rc = cg_enqueue(ctx, nullptr);
     if (rc) return rc;
     MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (cg_again(ctx)) {
+        if ((rc = cg_enqueue(ctx, nullptr, true))) return rc;
+        MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    }
     return cg_finish(ctx, st);
 }
 
