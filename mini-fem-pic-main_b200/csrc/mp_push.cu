@@ -230,9 +230,11 @@ __global__ void __launch_bounds__(PUSH_THREADS, 4) k_push_fp64(PushF64Args a) {
         if (i < n && cell >= 0) {
             const TetRec *t = a.tets + cell;
             // v += q_over_m*ef*dt ; x += v*dt  (src/mini-pic.cpp:291-295)
-            vx = __dadd_rn(vx, __dmul_rn(__dmul_rn(a.qm, __ldg(&t->ef[0])), a.dt));
-            vy = __dadd_rn(vy, __dmul_rn(__dmul_rn(a.qm, __ldg(&t->ef[1])), a.dt));
-            vz = __dadd_rn(vz, __dmul_rn(__dmul_rn(a.qm, __ldg(&t->ef[2])), a.dt));
+            double ef[4];  // and the volume
+            load32(t->ef, ef);
+            vx = __dadd_rn(vx, __dmul_rn(__dmul_rn(a.qm, ef[0]), a.dt));
+            vy = __dadd_rn(vy, __dmul_rn(__dmul_rn(a.qm, ef[1]), a.dt));
+            vz = __dadd_rn(vz, __dmul_rn(__dmul_rn(a.qm, ef[2]), a.dt));
             x = __dadd_rn(x, __dmul_rn(vx, a.dt));
             y = __dadd_rn(y, __dmul_rn(vy, a.dt));
             z = __dadd_rn(z, __dmul_rn(vz, a.dt));
@@ -267,22 +269,12 @@ __global__ void __launch_bounds__(PUSH_THREADS, 4) k_push_fp64(PushF64Args a) {
 // weight is within 1e-5 of zero the inside test and the exit face are decided
 // in FP64 with the reference's formula on x = x0 + r.  Walking to a new tet
 // re-bases r on that tet's vertex 0 (in FP64, rounded once to FP32).
-__device__ __forceinline__ void lambdas_fp32(const TetRec32 *__restrict__ t, float rx, float ry, float rz,
-                                             float lc[4]) {
-    const float4 gx = __ldg(reinterpret_cast<const float4 *>(t->gx));
-    const float4 gy = __ldg(reinterpret_cast<const float4 *>(t->gy));
-    const float4 gz = __ldg(reinterpret_cast<const float4 *>(t->gz));
-    lc[0] = 1.0f + fmaf(gx.x, rx, fmaf(gy.x, ry, gz.x * rz));
-    lc[1] = fmaf(gx.y, rx, fmaf(gy.y, ry, gz.y * rz));
-    lc[2] = fmaf(gx.z, rx, fmaf(gy.z, ry, gz.z * rz));
-    lc[3] = fmaf(gx.w, rx, fmaf(gy.w, ry, gz.w * rz));
-}
-
 __device__ __forceinline__ void load_x0(const double *__restrict__ x0, int cell, double &x, double &y, double &z) {
-    const double2 a = __ldg(reinterpret_cast<const double2 *>(x0 + 4ll * cell));
-    x = a.x;
-    y = a.y;
-    z = __ldg(x0 + 4ll * cell + 2);
+    double v[4];
+    load32(x0 + 4ll * cell, v);
+    x = v[0];
+    y = v[1];
+    z = v[2];
 }
 
 __global__ void __launch_bounds__(PUSH_THREADS, 4) k_push_mixed(PushF32Args a) {
@@ -322,15 +314,19 @@ __global__ void __launch_bounds__(PUSH_THREADS, 4) k_push_mixed(PushF32Args a) {
         float lc[4] = {0, 0, 0, 0};
         if (i < n && cell >= 0) {
             const TetRec32 *t = a.tets32 + cell;
-            vx = fmaf(a.qm_dt, __ldg(&t->ef[0]), vx);
-            vy = fmaf(a.qm_dt, __ldg(&t->ef[1]), vy);
-            vz = fmaf(a.qm_dt, __ldg(&t->ef[2]), vz);
+            float gxy[8], gzf[8];      // gradients along x, y | z, E field
+            load32(t->gx, gxy);
+            load32(t->gz, gzf);
+            vx = fmaf(a.qm_dt, gzf[4], vx);
+            vy = fmaf(a.qm_dt, gzf[5], vy);
+            vz = fmaf(a.qm_dt, gzf[6], vz);
             rx = fmaf(vx, a.dt, rx);
             ry = fmaf(vy, a.dt, ry);
             rz = fmaf(vz, a.dt, rz);
             for (;;) {
-                const TetRec32 *tc = a.tets32 + cell;
-                lambdas_fp32(tc, rx, ry, rz, lc);
+#pragma unroll
+                for (int k = 0; k < 4; k++) lc[k] = fmaf(gxy[k], rx, fmaf(gxy[4 + k], ry, gzf[k] * rz));
+                lc[0] += 1.0f;
                 float mn = fminf(fminf(lc[0], lc[1]), fminf(lc[2], lc[3]));
                 float mx = fmaxf(fmaxf(lc[0], lc[1]), fmaxf(lc[2], lc[3]));
                 // lambda > 1 implies another lambda < 0, so min alone picks the near-face cases
@@ -371,7 +367,7 @@ __global__ void __launch_bounds__(PUSH_THREADS, 4) k_push_mixed(PushF32Args a) {
                     state = 1;
                     break;
                 }
-                int nb = __ldg(&tc->cell_con[min_i]);
+                const int nb = __ldg(&a.tets32[cell].cell_con[min_i]);
                 if (nb < 0) {
                     state = 3;
                     cell = -1;
@@ -397,6 +393,9 @@ __global__ void __launch_bounds__(PUSH_THREADS, 4) k_push_mixed(PushF32Args a) {
                 rz = (float)((az - bz) + (double)rz);
                 cell = nb;
                 hops++;
+                const TetRec32 *tc = a.tets32 + cell;
+                load32(tc->gx, gxy);
+                load32(tc->gz, gzf);
             }
             if (state == 1) {
                 const int4 c4 = __ldg(reinterpret_cast<const int4 *>(a.tets32[cell].con));

@@ -9,21 +9,36 @@ namespace mp {
 
 constexpr double ONE_SIXTH = 1.0 / 6.0;
 
+// 32 bytes of a tet's record in one load (32-byte aligned, read-only).  A warp's
+// lanes read up to 32 records, and a load costs the L1 a pass per record whatever
+// its width: with 16-byte and scalar loads the mixed push kept the L1 at 74 % of
+// its rate.  Push kernel, before -> with these: mixed, 48M ions 1.23 -> 1.08 ms, 2M
+// 55 -> 51 us; FP64, 2M 85 -> 80 us.  (The mixed push's neighbours and nodes are
+// read when needed: loaded with the gradients they cost registers, 57 us at 2M.)
+__device__ __forceinline__ void load32(const double *p, double (&v)[4]) {
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
+__device__ __forceinline__ void load32(const float *p, float (&v)[8]) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+        : "l"(p));
+}
+__device__ __forceinline__ void load32(const int *p, int (&v)[8]) {
+    asm("ld.global.nc.v8.s32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+        : "l"(p));
+}
+
 // Numerators q_i = (1.0/6.0)*(alpha_i - x*beta_i + y*gamma_i - z*delta_i) of
 // the barycentric weights lambda_i = q_i/volume (src/meshes.h:84-85), in the
 // reference's order, every operation rounded on its own.
 __device__ __forceinline__ void numerators_fp64(const TetRec *__restrict__ t, double x, double y, double z,
                                                 double q[4]) {
-    const double2 *a2 = reinterpret_cast<const double2 *>(t->alpha);
-    const double2 *b2 = reinterpret_cast<const double2 *>(t->beta);
-    const double2 *g2 = reinterpret_cast<const double2 *>(t->gamma);
-    const double2 *d2 = reinterpret_cast<const double2 *>(t->delta);
     double al[4], be[4], ga[4], de[4];
-    double2 v;
-    v = __ldg(a2); al[0] = v.x; al[1] = v.y; v = __ldg(a2 + 1); al[2] = v.x; al[3] = v.y;
-    v = __ldg(b2); be[0] = v.x; be[1] = v.y; v = __ldg(b2 + 1); be[2] = v.x; be[3] = v.y;
-    v = __ldg(g2); ga[0] = v.x; ga[1] = v.y; v = __ldg(g2 + 1); ga[2] = v.x; ga[3] = v.y;
-    v = __ldg(d2); de[0] = v.x; de[1] = v.y; v = __ldg(d2 + 1); de[2] = v.x; de[3] = v.y;
+    load32(t->alpha, al);
+    load32(t->beta, be);
+    load32(t->gamma, ga);
+    load32(t->delta, de);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         double w = __dsub_rn(al[i], __dmul_rn(x, be[i]));
