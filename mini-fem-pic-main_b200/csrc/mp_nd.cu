@@ -17,8 +17,8 @@
 //   warp 17 (one lane) publisher: releases a finished tile's flag, so that only
 //                      it waits for the tile's stores.
 // Measured (B200, Newton step of the Lapack method, dense LDL^T before -> now): 567
-// unknowns 0.71 -> 0.16 ms, 8,379 15.6 -> 0.48 ms, 32,244 (mixed form) 41.4 ->
-// 1.33 ms.  The chain of diagonal blocks, 15 us a block (64 x 64 factor 8.4,
+// unknowns 0.70 -> 0.15 ms, 8,379 15.5 -> 0.46 ms, 32,244 (mixed form) 41.3 ->
+// 1.29 ms.  The chain of diagonal blocks, 15 us a block (64 x 64 factor 8.4,
 // products through the tile before it 3, hand-over between SMs 2; with 8 working
 // warps instead of 16, 17.7 us), bounds the
 // small meshes and the upper levels of the large ones; the FP64 tensor cores'
@@ -49,7 +49,7 @@ struct NdArgs {
     const int *perm, *ent_src;
     const unsigned short *ent_at;
     const double *kval, *FP, *b;
-    double *tile, *zd;
+    double *tile, *zd, *x;             // x: the solution by column, emptied here
     unsigned *flag;                    // [ntile] epoch of the tile's last forming
     unsigned *ctl;                     // ticket, abort
     unsigned long long *flags;
@@ -133,6 +133,38 @@ __device__ bool poll(const unsigned *f, unsigned epoch, unsigned *ctl_abort, uns
     for (unsigned i = 0;; i++) {
         if (ld_acquire(f) == epoch) return true;
         if ((i & 63) == 63 && *(volatile unsigned *)ctl_abort) return false;
+        if (i > POLL_LIMIT) {
+            give_up(ctl_abort, flags);
+            return false;
+        }
+    }
+}
+// A column's solution that is not formed yet: a NaN (a value that happens to carry
+// its bits is written as the canonical NaN), so that the values themselves are the
+// flag and a step of the backward solve is one trip through L2.
+constexpr unsigned long long EMPTY = 0xFFFFFFFFFFFFFFFFull;
+__device__ __forceinline__ unsigned long long ld_relaxed64(const double *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_value(double *p, double x) {
+    unsigned long long v = (unsigned long long)__double_as_longlong(x);
+    if (v == EMPTY) v = 0x7FF8000000000000ull;
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// Bounded wait until v[0], v[8], ..., v[56] are formed, all lanes of a warp alike.
+__device__ bool poll_values(const double *v, double (&x)[8], unsigned *ctl_abort, unsigned long long *flags) {
+    for (unsigned i = 0;; i++) {
+        bool ready = true;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const unsigned long long b = ld_relaxed64(v + 8 * k);
+            x[k] = __longlong_as_double((long long)b);
+            ready &= b != EMPTY;
+        }
+        if (__all_sync(0xffffffffu, ready)) return true;
+        if ((i & 63) == 63 && __any_sync(0xffffffffu, *(volatile unsigned *)ctl_abort)) return false;
         if (i > POLL_LIMIT) {
             give_up(ctl_abort, flags);
             return false;
@@ -461,13 +493,13 @@ __device__ __forceinline__ void trail_blocks(Smem &sm, int s, int first, int u0,
 
 // L D L^T of the 64 x 64 block in sm.c (lower part), warps 0-15: its inverse
 // (sm.inv, and in global memory at g), sm.d, sm.dinv, and z = L^-1 r (at gz; D and
-// 1/D beside it; `release` is arrived at after the first step).  Eight columns a
+// 1/D beside it; gx is emptied; `release` is arrived at after the first step).  Eight columns a
 // step.  Warp 0 runs the chain: it factors the 8 x 8 block, then forms the L rows
 // and updates the block that the next step factors, while the other warps do the
 // step's remaining rows and blocks and the inverse's next block row.  Latency-
 // bound, 2,000 clocks a step: the 8 x 8 block 1,150, the L rows 190, the update
 // 190, the rest barriers and the other warps' products (8 warps: 2,500 clocks).
-__device__ void factor64(Smem &sm, int warp, int lane, double *g, double *gz, unsigned long long *release,
+__device__ void factor64(Smem &sm, int warp, int lane, double *g, double *gz, double *gx, unsigned long long *release,
                          unsigned long long *flags) {
     auto z_rows = [&](int w) {
         const double zr = sum_quad(row_dot(sm.inv, sm.r, 8, w, lane));
@@ -547,6 +579,8 @@ __device__ void factor64(Smem &sm, int warp, int lane, double *g, double *gz, un
     } else if (warp < 5) {
         const int i = 32 * (warp - 1) + lane;
         gz[T + i] = i < T ? sm.d[i] : sm.dinv[i - T];
+    } else if (warp < 7) {
+        gx[32 * (warp - 5) + lane] = __longlong_as_double((long long)EMPTY);
     }
 }
 
@@ -823,7 +857,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_nd_factor(NdArgs a) {
             if (rw >= 0 && (lane & 3) == 0) sm.r[8 * rw + (lane >> 2)] -= rs;
             sync_work();
         }
-        factor64(sm, warp, lane, a.tile + (size_t)out * TT, a.zd + (size_t)J * ZD, fused ? &sm.empty[s] : nullptr,
+        factor64(sm, warp, lane, a.tile + (size_t)out * TT, a.zd + (size_t)J * ZD, a.x + (size_t)J * T, fused ? &sm.empty[s] : nullptr,
                  a.flags);
         publish(out, -1);
     }
@@ -861,7 +895,11 @@ struct SolveSmem {
 // z_J - sum_I L_IJ^T x_I), which also adds to or sets y.  A column is a task,
 // taken by ticket in the elimination order or its reverse; the producer
 // streams the column's tiles, which do not depend on the solve, ahead of the
-// values the others wait for.
+// values the others wait for.  Latency-bound: a chain of columns.  Backward, the
+// values themselves are polled (no flag and no fence on the way) and z, D^-1 and
+// the unknowns' numbers are read when a column starts: 16.6 -> 11.7 us at 567
+// unknowns, 58 -> 40 at 8,379, 137 -> 90 at 32,244.  The launch before a
+// backward one (a factor, a forward solve) empties x.
 template <bool BACK>
 __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -912,25 +950,41 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
         }
         return;
     }
-    const double *src = BACK ? a.x : a.zd;   // the values of solved columns
-    const int pitch = BACK ? T : ZD;
     // forward: warp w holds rows 8w .. 8w + 7, backward columns
-    double s0 = 0.0, s1 = 0.0;
+    double s0 = 0.0, s1 = 0.0, rhs0 = 0.0, rhs1 = 0.0;
+    int at = -1, u0 = -1, u1 = -1;            // the column under way; its lane's unknowns
     for (unsigned it = 0;; it++) {
         const int s = it % SOLVE_STAGES;
         bool ok = bar_wait(&sm.full[s], (it / SOLVE_STAGES) & 1, &sm.abort);
         const int J = sm.col[s], last = sm.last[s];
+        if (ok && J >= 0 && J != at) {
+            // what the column's end needs and does not depend on the others
+            at = J;
+            if (BACK && lane < 4) {
+                const double *z = a.zd + (size_t)J * ZD + 8 * warp + lane;
+                rhs0 = __ldcg(z) * __ldcg(z + 2 * T);
+                rhs1 = __ldcg(z + 4) * __ldcg(z + 2 * T + 4);
+                u0 = a.perm[J * T + 8 * warp + lane];
+                u1 = a.perm[J * T + 8 * warp + lane + 4];
+            }
+            if (!BACK && (lane & 3) == 0) {
+                u0 = a.perm[J * T + 8 * warp + (lane >> 2)];
+                rhs0 = u0 >= 0 ? a.b[u0] : 0.0;
+            }
+        }
         if (ok && J >= 0 && !last) {
             const int o = sm.other[s];
-            if (lane == 0) ok = poll(a.flag + o, a.epoch, a.ctl + 1, a.flags);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            __syncwarp();
-            const double *v = src + (size_t)o * pitch;
             double x[16];
-            if (BACK) {
+            if constexpr (BACK) {
+                double w[8];
+                ok = poll_values(a.x + (size_t)o * T + (lane >> 2), w, a.ctl + 1, a.flags);
 #pragma unroll
-                for (int k = 0; k < 8; k++) x[k] = __ldcg(v + 8 * k + (lane >> 2));
+                for (int k = 0; k < 8; k++) x[k] = w[k];
             } else {
+                if (lane == 0) ok = poll(a.flag + o, a.epoch, a.ctl + 1, a.flags);
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                __syncwarp();
+                const double *v = a.zd + (size_t)o * ZD;
 #pragma unroll
                 for (int k = 0; k < 16; k++) x[k] = __ldcg(v + 4 * k + (lane & 3));
             }
@@ -963,16 +1017,13 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
                 s1 += __shfl_xor_sync(0xffffffffu, s1, o);
             }
             if (lane < 4) {
-                const double *z = a.zd + (size_t)J * ZD;
-                const int c = 8 * warp + lane;
-                sm.v[c] = __ldcg(z + c) * __ldcg(z + 2 * T + c) - s0;
-                sm.v[c + 4] = __ldcg(z + c + 4) * __ldcg(z + 2 * T + c + 4) - s1;
+                sm.v[8 * warp + lane] = rhs0 - s0;
+                sm.v[8 * warp + lane + 4] = rhs1 - s1;
             }
         } else {
             s0 = sum_quad(s0 + s1);
             if ((lane & 3) == 0) {
-                const int r = 8 * warp + (lane >> 2), u = a.perm[J * T + r];
-                sm.v[r] = u >= 0 ? a.b[u] - s0 : 0.0;
+                sm.v[8 * warp + (lane >> 2)] = u0 >= 0 ? rhs0 - s0 : 0.0;
             }
         }
         sync_work<SOLVE_WORK>();
@@ -990,22 +1041,21 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
                 s1 += __shfl_xor_sync(0xffffffffu, s1, o);
             }
             if (lane < 4) {
-                const int c = 8 * warp + lane;
-                a.x[(size_t)J * T + c] = s0;
-                a.x[(size_t)J * T + c + 4] = s1;
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int u = a.perm[J * T + c + 4 * e];
-                    if (u >= 0) a.y[u] = a.add ? a.y[u] + (e ? s1 : s0) : (e ? s1 : s0);
-                }
+                st_value(a.x + (size_t)J * T + 8 * warp + lane, s0);
+                st_value(a.x + (size_t)J * T + 8 * warp + lane + 4, s1);
+                if (u0 >= 0) a.y[u0] = a.add ? a.y[u0] + s0 : s0;
+                if (u1 >= 0) a.y[u1] = a.add ? a.y[u1] + s1 : s1;
             }
         } else {
             const double zr = sum_quad(row_dot(sm.stage[s], sm.v, warp + 1, warp, lane));
-            if ((lane & 3) == 0) a.zd[(size_t)J * ZD + 8 * warp + (lane >> 2)] = zr;
+            if ((lane & 3) == 0) {
+                a.zd[(size_t)J * ZD + 8 * warp + (lane >> 2)] = zr;
+                a.x[(size_t)J * T + 8 * warp + (lane >> 2)] = __longlong_as_double((long long)EMPTY);
+            }
         }
         s0 = s1 = 0.0;
         sync_work<SOLVE_WORK>();
-        if (t == 0) st_release(a.flag + J, a.epoch);
+        if (!BACK && t == 0) st_release(a.flag + J, a.epoch);
         if (lane == 0) bar_arrive(&sm.empty[s]);
     }
 }
@@ -1021,7 +1071,7 @@ struct NdState {
     const unsigned short *ent_at = nullptr;
     int ntask = 0;
     double *tile = nullptr, *zd = nullptr, *x = nullptr;
-    unsigned *flag = nullptr;          // tiles (and scratch ones), then [2][ncol] forward and backward columns
+    unsigned *flag = nullptr;          // tiles (and scratch ones), then the forward columns
     size_t words = 0;
     unsigned *ctl = nullptr;           // [3][2] ticket and abort word of a factor, a forward and a backward launch
     unsigned epoch = 0;
@@ -1106,7 +1156,7 @@ int nd_prepare(mp_ctx *ctx, bool mixed, bool *usable) {
             MP_CUDA(ctx, cudaMalloc(&s->x, sizeof(double) * (size_t)p.ncol * T));
             // the blocks above an inverse's diagonal stay zero
             MP_CUDA(ctx, cudaMemsetAsync(s->tile, 0, sizeof(double) * (size_t)p.ntile * TT, ctx->stream));
-            s->words = (size_t)p.ntile + p.nscratch + 2 * (size_t)p.ncol;
+            s->words = (size_t)p.ntile + p.nscratch + (size_t)p.ncol;
             MP_CUDA(ctx, cudaMalloc(&s->flag, sizeof(unsigned) * s->words));
             MP_CUDA(ctx, cudaMemsetAsync(s->flag, 0, sizeof(unsigned) * s->words, ctx->stream));
             MP_CUDA(ctx, cudaMalloc(&s->ctl, sizeof(unsigned) * 8));
@@ -1138,7 +1188,7 @@ static int nd_launch_solve(mp_ctx *ctx, NdState *s, bool back, const double *b, 
     a.zd = s->zd;
     a.x = s->x;
     a.y = y;
-    a.flag = s->flag + p.ntile + p.nscratch + (back ? p.ncol : 0);
+    a.flag = s->flag + p.ntile + p.nscratch;
     a.ctl = s->ctl + (back ? 4 : 2);
     a.flags = ctx->counters + C_FLAGS;
     a.ncol = p.ncol;
@@ -1185,6 +1235,7 @@ int nd_factor_solve(mp_ctx *ctx, const double *b, double *y, bool control_cleare
     a.b = b;
     a.tile = s->tile;
     a.zd = s->zd;
+    a.x = s->x;
     a.flag = s->flag;
     a.ctl = s->ctl;
     a.flags = ctx->counters + C_FLAGS;
