@@ -14,7 +14,7 @@ Kuhn box minus the centred r = 0.02 m sphere held at -10 V (189,972 tets,
 steady state (48.3M inside the domain: drift 7 km/s + 0.1 eV Maxwellian),
 spwt 0.2, dt 5e-8 s, the reference's per-face injection counts every step
 (about 175k ions), a tet re-sort every 10 steps.  A step is InjectIons ->
-MoveParticles -> computePhi (Lapack method: one Newton step, dense LDL^T) ->
+MoveParticles -> computePhi (Lapack method: one Newton step, sparse LDL^T) ->
 updateEf.  The synthetic seeded population stands in for a physical run.
 
 value        particle-steps/s of the mixed form's whole step (device-resident:
@@ -186,14 +186,19 @@ def kernel_roofline(ctx, form, pk, step_ms_total, sustained=True, neq=0):
     classes = {k: ctx.kernel_timing(k) for k in KT_NAMES if mp.KT_TIMED >> k & 1}
     share = {KT_NAMES[k]: {"launches": v["launches"], "ms": v["ms"], "share_of_step": v["ms"] / step_ms_total}
              for k, v in classes.items()}
-    share["diagonal_factor + panel + the rest"] = {
+    share["the rest"] = {
         "ms": step_ms_total - sum(v["ms"] for v in classes.values()),
-        "what": "not bracketed by events in the timed run (hundreds of small launches a step)"}
+        "what": "not bracketed by events in the timed run (small launches, read-backs; a dense "
+                "factorization's diagonal factors and panels)"}
     top = max(classes, key=lambda k: classes[k]["ms"])
     v = classes[top]
     terms = mixed_terms(neq)
+    # one factorization launch a step: the sparse direct solver
+    sparse = classes[mp.KT_UPDATE]["launches"] <= classes[mp.KT_PUSH]["launches"]
     kname = KT_KERNEL[top][form]
-    if top == mp.KT_UPDATE and form == mp.MIXED:
+    if sparse and top in (mp.KT_UPDATE, mp.KT_TRSV):
+        kname = "k_nd_factor (FP64 mma.sync m8n8k4)" if top == mp.KT_UPDATE else "k_nd_solve"
+    elif top == mp.KT_UPDATE and form == mp.MIXED:
         kname = ("tc::k_update_tc<1> (3xTF32, tcgen05 kind::tf32)" if terms == mp.MIXED_TF32X3 else
                  "tc::k_update_tc_tma<2> (FP16 operands, tcgen05 kind::f16, old values of A moved by TMA)")
     out = {"kernel": kname, "class": KT_NAMES[top], "launches": v["launches"],
@@ -207,6 +212,13 @@ def kernel_roofline(ctx, form, pk, step_ms_total, sustained=True, neq=0):
         bpp = 52.0 if form == mp.FP64 else 28.0
         out["traffic"] = TRAFFIC_PER_UNIT[key] * v["work"] / bpp / max(v["launches"], 1)
         out["traffic_source"] = "ncu DRAM bytes per particle (20^3 box, 2M ions) x this launch's particles"
+    elif top == mp.KT_UPDATE and sparse:
+        ach = v["work"] / (v["ms"] * 1e-3) / 1e12
+        out.update(bound="latency (the chain of 64 x 64 diagonal blocks) and tensor (FP64)", achieved=ach,
+                   peak=FP64_TENSOR_TFLOPS, unit="TFLOP/s", frac=ach / FP64_TENSOR_TFLOPS,
+                   peak_kind="FP64 tensor pipe: 26.4 TFLOP/s at 76.6 % pipe activity in one ncu capture "
+                             "(profiles/k_update_f64_kuhn20_newton.md); no FP64 peak was measured",
+                   algorithmic="2 flops per multiply-add of the sparse factor's tile products")
     elif top == mp.KT_UPDATE and form == mp.FP64:
         ach = v["work"] / (v["ms"] * 1e-3) / 1e12
         out.update(bound="tensor (FP64)", achieved=ach, peak=FP64_TENSOR_TFLOPS, unit="TFLOP/s",
@@ -854,8 +866,8 @@ def main():
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64",
             "data": "synthetic (seeded Kuhn-box ions at steady state; device injection with the reference's counts)",
             "config": conf,
-            "form": "mixed: FP32 tet-relative particles, FP64 near-face test and density, %s tcgen05 LDL^T "
-                    "with FP64 refinement" % ("FP16-operand" if mixed_terms(h["neq"]) == mp.MIXED_FP16 else "3xTF32"),
+            "form": "mixed: FP32 tet-relative particles, FP64 near-face test and density, sparse FP64 LDL^T "
+                    "with FP64 refinement",
             "parallelism": f"particles sharded x{world}, density all-reduce, field solve replicated"
             if world > 1 else "1 GPU",
             "l2": f"inputs larger than L2 (the particle arrays); {FLUSH_BYTES >> 20} MiB written between steps",

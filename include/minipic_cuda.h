@@ -84,11 +84,13 @@ enum { MP_FE_STORAGE_DENSE = 0, MP_FE_STORAGE_SPARSE = 1 };
 
 /* Arithmetic forms. FP64 is the reference's method bit for bit on the particle
  * side; MIXED stores particles as FP32 offsets from the owning tet's vertex 0
- * (FP64 near-face re-test, FP64 density accumulators) and factors the Newton
- * Jacobian in TF32 on the tensor cores with FP64 iterative refinement. */
+ * (FP64 near-face re-test, FP64 density accumulators) and refines the Newton
+ * solve to ||G - J y|| <= 1e-14 ||G|| in FP64.  Both factor the sparse Jacobian
+ * in FP64 where that is the faster way; the dense factor is FP64 or, in the mixed
+ * form, FP32 with tensor-core updates. */
 enum { MP_FORM_FP64 = 0, MP_FORM_MIXED = 1 };
 
-/* Tensor-core arithmetic of the mixed form's FP32 factorization: one TF32
+/* Tensor-core arithmetic of the mixed form's dense FP32 factorization: one TF32
  * product per term, or the 3xTF32 split (hi*hi + hi*lo + lo*hi, about FP32
  * accuracy; fewer FP64 refinement iterations). */
 enum { MP_MIXED_AUTO = 0, MP_MIXED_TF32 = 1, MP_MIXED_FP16 = 2, MP_MIXED_TF32X3 = 3 };
@@ -207,9 +209,10 @@ int mp_set_particle_form(mp_ctx *ctx, int form);
  *                    FP16 the factorization is redone with TF32 operands;
  *   MP_MIXED_TF32X3  hi/lo split, three TF32 products a term (about FP32
  *                    accuracy, fewer refinement solves);
- *   MP_MIXED_AUTO    the default: TF32X3 below MP_MIXED_FP16_FROM unknowns,
- *                    where the refinement solves cost more than the trailing
- *                    update saves, FP16 from there on.
+ *   MP_MIXED_AUTO    the default: the sparse FP64 factorization where K has the
+ *                    mesh's pattern and that is faster; else TF32X3 below
+ *                    MP_MIXED_FP16_FROM unknowns, where the refinement solves
+ *                    cost more than the trailing update saves, FP16 from there on.
  * Either way the solve is refined in FP64 to the same tolerance.  No
  * reference counterpart: the reference's dsysv_ call (src/FESolver.cpp:528-558)
  * is FP64 throughout. */
@@ -237,10 +240,11 @@ int mp_kernel_launches(mp_ctx *ctx, int64_t *n);
  * them out).  work: algorithmic bytes for MP_KT_PUSH ((particles before + after
  * the push) x the form's bytes per particle, 52 FP64 / 28 mixed), algorithmic
  * flops for MP_KT_UPDATE (2 per multiply-add of the trailing update's lower
- * triangle; the 3xTF32 split issues three tensor-core products per term and
- * counts once), 0 for the latency-bound classes. */
+ * triangle, or of the sparse factorization's tile products; the 3xTF32 split
+ * issues three tensor-core products per term and counts once), 0 for the
+ * latency-bound classes. */
 enum { MP_KT_PUSH = 0,    /* the push + walk + scatter kernel */
-       MP_KT_UPDATE = 1,  /* trailing updates of the LDL^T: tcgen05 (mixed) or register-tiled FP64 */
+       MP_KT_UPDATE = 1,  /* the sparse factorization, or a dense one's trailing updates */
        MP_KT_DIAG = 2,    /* diagonal-block factorizations */
        MP_KT_PANEL = 3,   /* panels, in-panel column updates and operand splits */
        MP_KT_TRSV = 4     /* triangular solves */ };

@@ -20,9 +20,9 @@
 // unknowns 0.70 -> 0.15 ms, 8,379 15.5 -> 0.46 ms, 32,244 (mixed form) 41.3 ->
 // 1.29 ms.  The chain of diagonal blocks, 15 us a block (64 x 64 factor 8.4,
 // products through the tile before it 3, hand-over between SMs 2; with 8 working
-// warps instead of 16, 17.7 us), bounds the
-// small meshes and the upper levels of the large ones; the FP64 tensor cores'
-// rate (64 multiply-adds a cycle and SM) and the tasks' own latency the lower levels.
+// warps instead of 16, 17.7 us), bounds the small meshes and the upper levels of
+// the large ones; the FP64 tensor cores' rate (64 multiply-adds a cycle and SM) and
+// the tasks' own latency the lower levels.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

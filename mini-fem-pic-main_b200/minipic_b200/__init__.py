@@ -487,8 +487,9 @@ class Context:
 
     def set_mixed_factor(self, mode):
         """MIXED_AUTO (default), MIXED_TF32, MIXED_FP16 or MIXED_TF32X3: tensor-core arithmetic
-        of the mixed-form factorization (AUTO: TF32X3 below 16,384 unknowns, FP16 from there;
-        FP16: the trailing updates on scaled FP16 copies of their operands)."""
+        of the mixed form's dense factorization (AUTO: the sparse FP64 factorization where it is
+        faster, else TF32X3 below 16,384 unknowns, FP16 from there; FP16: the trailing updates on
+        scaled FP16 copies of their operands)."""
         self._c(lib().mp_set_mixed_factor(self.h, mode))
 
     def set_sort_period(self, steps):

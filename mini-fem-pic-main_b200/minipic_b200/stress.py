@@ -2,14 +2,14 @@
 centred r = 0.02 m sphere held at -10 V (371,004 tets, 67,298 nodes, 62,788
 unknowns; the dense FP64 K is 31.6 GB), about 193M O+ ions (spwt 0.05) with a
 tet re-sort every 10 steps, the mixed-precision step (FP32 tet-relative
-particles, tcgen05 LDL^T on FP16 operands with FP64 refinement), the adjoint of K = 10
+particles, sparse LDL^T with FP64 refinement), the adjoint of K = 10
 push + scatter steps with checkpoints every 5 on the whole population, and the
 FP64 form of the same steps beside it.
 
-Memory plan (one B200, 180 GB): the mixed run holds K (31.6 GB), its FP32
-factor (15.8 GB), the particles (two buffers, 60 B a slot, 24 GB) and then the
-adjoint's slots (inputs, two checkpoints and outcomes, about 160 B a slot,
-31 GB); the FP64 run afterwards holds K, the FP64 J (31.6 GB) and the particles.
+Memory plan (one B200, 180 GB): either run holds the dense K (31.6 GB), the
+sparse factor and the particles (two buffers of 60 B a slot, 24 GB);
+the mixed one then the adjoint's slots (inputs, two checkpoints and outcomes,
+about 160 B a slot, 31 GB).
 The two never share the device.  The population is generated and appended in
 chunks of 16M ions, so the host never holds it whole.
 
@@ -113,8 +113,7 @@ def run(args, device, torch, pk):
     keep_m = []
     rm = _steps(c, mp.MIXED, cfg, deck, steps, warmup, torch, device, keep_m)
     out["mixed"] = _summary(rm, c, pk)
-    out["mixed"]["refined_newton"] = ("tcgen05 LDL^T (FP16-operand trailing updates from %d unknowns, 3xTF32 below), "
-                                      "FP64 refinement to ||r|| <= 1e-14 ||G||" % mp.MIXED_FP16_FROM)
+    out["mixed"]["refined_newton"] = "sparse FP64 LDL^T, FP64 refinement to ||r|| <= 1e-14 ||G||"
     free, total = torch.cuda.mem_get_info(device)
     out["mixed"]["device_memory_used_GB"] = (total - free) / 1e9
     # adjoint of K push + scatter steps over the whole population, phi held at the last step's
