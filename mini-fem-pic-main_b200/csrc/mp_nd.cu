@@ -139,9 +139,9 @@ __device__ bool poll(const unsigned *f, unsigned epoch, unsigned *ctl_abort, uns
         }
     }
 }
-// A column's solution that is not formed yet: a NaN (a value that happens to carry
-// its bits is written as the canonical NaN), so that the values themselves are the
-// flag and a step of the backward solve is one trip through L2.
+// A column's solution, or z, that is not formed yet: a NaN (a value that happens to
+// carry its bits is written as the canonical NaN), so that the values themselves are
+// the flag and a step of a triangular solve is one trip through L2.
 constexpr unsigned long long EMPTY = 0xFFFFFFFFFFFFFFFFull;
 __device__ __forceinline__ unsigned long long ld_relaxed64(const double *p) {
     unsigned long long v;
@@ -153,13 +153,14 @@ __device__ __forceinline__ void st_value(double *p, double x) {
     if (v == EMPTY) v = 0x7FF8000000000000ull;
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-// Bounded wait until v[0], v[8], ..., v[56] are formed, all lanes of a warp alike.
-__device__ bool poll_values(const double *v, double (&x)[8], unsigned *ctl_abort, unsigned long long *flags) {
+// Bounded wait until v[0], v[STEP], ..., v[(N - 1) STEP] are formed, all lanes of a warp alike.
+template <int N, int STEP>
+__device__ bool poll_values(const double *v, double (&x)[N], unsigned *ctl_abort, unsigned long long *flags) {
     for (unsigned i = 0;; i++) {
         bool ready = true;
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const unsigned long long b = ld_relaxed64(v + 8 * k);
+        for (int k = 0; k < N; k++) {
+            const unsigned long long b = ld_relaxed64(v + STEP * k);
             x[k] = __longlong_as_double((long long)b);
             ready &= b != EMPTY;
         }
@@ -877,10 +878,9 @@ struct SolveArgs {
     const double *tile, *b;
     double *zd, *x;                    // z (forward result), x [ncol][64]
     double *y;                         // solution by unknown
-    unsigned *flag, *ctl;
+    unsigned *ctl;
     unsigned long long *flags;
     int ncol, add;
-    unsigned epoch;
 };
 
 struct SolveSmem {
@@ -895,11 +895,12 @@ struct SolveSmem {
 // z_J - sum_I L_IJ^T x_I), which also adds to or sets y.  A column is a task,
 // taken by ticket in the elimination order or its reverse; the producer
 // streams the column's tiles, which do not depend on the solve, ahead of the
-// values the others wait for.  Latency-bound: a chain of columns.  Backward, the
-// values themselves are polled (no flag and no fence on the way) and z, D^-1 and
-// the unknowns' numbers are read when a column starts: 16.6 -> 11.7 us at 567
-// unknowns, 58 -> 40 at 8,379, 137 -> 90 at 32,244.  The launch before a
-// backward one (a factor, a forward solve) empties x.
+// values the others wait for.  Latency-bound: a chain of columns.  The values
+// themselves are polled (no flag and no fence on the way), and what a column's end
+// needs besides is read when the column starts: backward 16.6 -> 11.7 us at 567
+// unknowns, 58 -> 40 at 8,379, 137 -> 90 at 32,244; forward 128 -> 103.  A launch
+// empties what the next one fills: a factor or a forward solve x, a backward
+// solve z.
 template <bool BACK>
 __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -974,24 +975,13 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
         }
         if (ok && J >= 0 && !last) {
             const int o = sm.other[s];
-            double x[16];
-            if constexpr (BACK) {
-                double w[8];
-                ok = poll_values(a.x + (size_t)o * T + (lane >> 2), w, a.ctl + 1, a.flags);
-#pragma unroll
-                for (int k = 0; k < 8; k++) x[k] = w[k];
-            } else {
-                if (lane == 0) ok = poll(a.flag + o, a.epoch, a.ctl + 1, a.flags);
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                __syncwarp();
-                const double *v = a.zd + (size_t)o * ZD;
-#pragma unroll
-                for (int k = 0; k < 16; k++) x[k] = __ldcg(v + 4 * k + (lane & 3));
-            }
+            double x[BACK ? 8 : 16];
+            if constexpr (BACK) ok = poll_values<8, 8>(a.x + (size_t)o * T + (lane >> 2), x, a.ctl + 1, a.flags);
+            else ok = poll_values<16, 4>(a.zd + (size_t)o * ZD + (lane & 3), x, a.ctl + 1, a.flags);
 #pragma unroll
             for (int k = 0; k < 8; k++) {
                 const double2 l = frag(sm.stage[s] + (BACK ? warp * 512 + k * 64 : k * 512 + warp * 64), lane);
-                if (BACK) {
+                if constexpr (BACK) {
                     s0 = fma(l.x, x[k], s0);
                     s1 = fma(l.y, x[k], s1);
                 } else {
@@ -1043,19 +1033,20 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
             if (lane < 4) {
                 st_value(a.x + (size_t)J * T + 8 * warp + lane, s0);
                 st_value(a.x + (size_t)J * T + 8 * warp + lane + 4, s1);
+                double *z = a.zd + (size_t)J * ZD + 8 * warp + lane;  // for the next forward solve
+                z[0] = z[4] = __longlong_as_double((long long)EMPTY);
                 if (u0 >= 0) a.y[u0] = a.add ? a.y[u0] + s0 : s0;
                 if (u1 >= 0) a.y[u1] = a.add ? a.y[u1] + s1 : s1;
             }
         } else {
             const double zr = sum_quad(row_dot(sm.stage[s], sm.v, warp + 1, warp, lane));
             if ((lane & 3) == 0) {
-                a.zd[(size_t)J * ZD + 8 * warp + (lane >> 2)] = zr;
+                st_value(a.zd + (size_t)J * ZD + 8 * warp + (lane >> 2), zr);
                 a.x[(size_t)J * T + 8 * warp + (lane >> 2)] = __longlong_as_double((long long)EMPTY);
             }
         }
         s0 = s1 = 0.0;
         sync_work<SOLVE_WORK>();
-        if (!BACK && t == 0) st_release(a.flag + J, a.epoch);
         if (lane == 0) bar_arrive(&sm.empty[s]);
     }
 }
@@ -1071,7 +1062,7 @@ struct NdState {
     const unsigned short *ent_at = nullptr;
     int ntask = 0;
     double *tile = nullptr, *zd = nullptr, *x = nullptr;
-    unsigned *flag = nullptr;          // tiles (and scratch ones), then the forward columns
+    unsigned *flag = nullptr;          // tiles (and scratch ones)
     size_t words = 0;
     unsigned *ctl = nullptr;           // [3][2] ticket and abort word of a factor, a forward and a backward launch
     unsigned epoch = 0;
@@ -1156,7 +1147,7 @@ int nd_prepare(mp_ctx *ctx, bool mixed, bool *usable) {
             MP_CUDA(ctx, cudaMalloc(&s->x, sizeof(double) * (size_t)p.ncol * T));
             // the blocks above an inverse's diagonal stay zero
             MP_CUDA(ctx, cudaMemsetAsync(s->tile, 0, sizeof(double) * (size_t)p.ntile * TT, ctx->stream));
-            s->words = (size_t)p.ntile + p.nscratch + (size_t)p.ncol;
+            s->words = (size_t)p.ntile + p.nscratch;
             MP_CUDA(ctx, cudaMalloc(&s->flag, sizeof(unsigned) * s->words));
             MP_CUDA(ctx, cudaMemsetAsync(s->flag, 0, sizeof(unsigned) * s->words, ctx->stream));
             MP_CUDA(ctx, cudaMalloc(&s->ctl, sizeof(unsigned) * 8));
@@ -1188,12 +1179,10 @@ static int nd_launch_solve(mp_ctx *ctx, NdState *s, bool back, const double *b, 
     a.zd = s->zd;
     a.x = s->x;
     a.y = y;
-    a.flag = s->flag + p.ntile + p.nscratch;
     a.ctl = s->ctl + (back ? 4 : 2);
     a.flags = ctx->counters + C_FLAGS;
     a.ncol = p.ncol;
     a.add = add;
-    a.epoch = s->epoch;
     const int grid = std::min(ctx->sm_count, p.ncol);
     const int mk = kt_begin(ctx, MP_KT_TRSV, 0);
     if (back) k_nd_solve<true><<<grid, SOLVE_THREADS, sizeof(SolveSmem), ctx->stream>>>(a), ++ctx->launches;

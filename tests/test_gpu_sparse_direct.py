@@ -166,3 +166,23 @@ def test_step_terms_bitwise(tmp_path, n, sphere, method):
     y, now, uh, g = (ctx.fe_get(k) for k in ("y", "d", "uh", "g"))
     assert np.array_equal(now, d - y)
     assert np.array_equal(uh, np.where(ID >= 0, g + now[ID], g))
+
+
+def test_refinement(tmp_path):
+    """Right-hand sides whose solution is far larger (inverse iteration, J's smoothest
+    modes): the mixed form refines, by forward and backward solves with the factor."""
+    kd, path = make_deck(tmp_path, 16)
+    ctx = context(mp.Deck.load(path))
+    b = state(ctx, 7)
+    ctx.build_j(mp.LAPACK)
+    J = ctx.fe_get("J")
+    most = 0
+    for _ in range(8):
+        ctx.build_j(mp.LAPACK)
+        st = ctx.solve_linear(mp.LAPACK, mp.MIXED, b=b)
+        y = ctx.fe_get("y")
+        assert np.linalg.norm(b - J @ y) <= 1e-13 * np.linalg.norm(b)
+        most = max(most, st.linear_iterations)
+        last, b = b, y / np.linalg.norm(y)
+    assert most > 1
+    assert rel(y, np.linalg.solve(J, last)) < TOL
