@@ -75,8 +75,8 @@ struct AdjState {
     bool path_valid = false;
     // mesh-sized
     double *nx = nullptr;       // [n_tets][12]
-    double *ef = nullptr;       // [n_tets][3] ef of the tape's phi
-    double *def = nullptr;      // [n_tets][3] tangent ef / reverse Ebar
+    double *ef = nullptr;       // [n_tets][4] ef of the tape's phi, and the volume
+    double *def = nullptr;      // [n_tets][4] tangent ef / [n_tets][3] reverse Ebar
     unsigned char *wall = nullptr;  // [n_tets] bit i: face opposite vertex i is a wall face
     double *nodes_a = nullptr, *nodes_b = nullptr;  // [n_nodes] scratch
     double *scal = nullptr;     // device [4]: flux, vdbar, dflux, spare; [4]: slots by outcome (KIND_*), 64-bit counts
@@ -111,7 +111,8 @@ __device__ __forceinline__ Slot start_slot(const AdjArgs &a, long long p) {
     Slot s{a.px[p], a.py[p], a.pz[p], a.vx[p], a.vy[p], a.vz[p], a.cell0[p]};
     if (a.inj[p]) {
         // vel = normal*ion_velocity (+ thermal part); vel -= charge/mass*ef*(0.5*dt)
-        const double *e = a.ef + 3 * s.cell;
+        double e[4];
+        load32(a.ef + 4 * (long long)s.cell, e);
         const double hdt = 0.5 * a.dt;
         s.vx = __dsub_rn(__dadd_rn(__dmul_rn(a.dir0, a.vd), s.vx), __dmul_rn(__dmul_rn(a.qm, e[0]), hdt));
         s.vy = __dsub_rn(__dadd_rn(__dmul_rn(a.dir1, a.vd), s.vy), __dmul_rn(__dmul_rn(a.qm, e[1]), hdt));
@@ -120,20 +121,24 @@ __device__ __forceinline__ Slot start_slot(const AdjArgs &a, long long p) {
     return s;
 }
 
-// v += q_over_m*ef*dt ; x += v*dt  (src/mini-pic.cpp:291-295), unfused
-__device__ __forceinline__ void kick_drift(Slot &s, const double *ef, double qm, double dt) {
-    const double *e = ef + 3 * s.cell;
+// v += q_over_m*ef*dt ; x += v*dt  (src/mini-pic.cpp:291-295), unfused.  Returns the tet's volume.
+__device__ __forceinline__ double kick_drift(Slot &s, const double *ef, double qm, double dt) {
+    double e[4];
+    load32(ef + 4 * (long long)s.cell, e);
     s.vx = __dadd_rn(s.vx, __dmul_rn(__dmul_rn(qm, e[0]), dt));
     s.vy = __dadd_rn(s.vy, __dmul_rn(__dmul_rn(qm, e[1]), dt));
     s.vz = __dadd_rn(s.vz, __dmul_rn(__dmul_rn(qm, e[2]), dt));
     s.x = __dadd_rn(s.x, __dmul_rn(s.vx, dt));
     s.y = __dadd_rn(s.y, __dmul_rn(s.vy, dt));
     s.z = __dadd_rn(s.z, __dmul_rn(s.vz, dt));
+    return e[3];
 }
 
 // Cell update of step k: the reference walk, or the recorded path when pinned.
-// Returns KIND_*; lc holds the end cell's coordinates when walked and inside.
-__device__ __forceinline__ int move_cell(const AdjArgs &a, Slot &s, int k, long long p, double lc[4]) {
+// Returns KIND_*.  vol: the volume of the tet it starts in.  EXACT_CMP as for the
+// walk: the cells alone are wanted here, and its weights differ in the last bits.
+template <bool EXACT_CMP>
+__device__ __forceinline__ int move_cell(const AdjArgs &a, Slot &s, int k, long long p, double vol) {
     if (a.pinned) {
         const int c = a.path[(long long)k * a.cap + p];
         if (c >= 0) {
@@ -143,7 +148,8 @@ __device__ __forceinline__ int move_cell(const AdjArgs &a, Slot &s, int k, long 
         return c == PATH_EXIT_WALL ? KIND_WALL : c == PATH_EXIT_OTHER ? KIND_OTHER : KIND_LIMIT;
     }
     int cell = s.cell, hops = 0, face = 0;
-    const int w = walk_fp64(a.tets, cell, s.x, s.y, s.z, lc, a.walk_limit, hops, &face);
+    double lc[4];
+    const int w = walk_fp64<EXACT_CMP>(a.tets, cell, s.x, s.y, s.z, vol, lc, a.walk_limit, hops, &face);
     int r;
     if (w == 1) {
         s.cell = cell;
@@ -197,7 +203,7 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
 }
 
 __global__ void k_adj_ef(int n_tets, const int *__restrict__ con, const double *__restrict__ nx,
-                         const double *__restrict__ phi, double *ef) {
+                         const double *__restrict__ phi, const TetRec *__restrict__ tets, double *ef) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n_tets) return;
     double f[3] = {0, 0, 0};
@@ -205,7 +211,8 @@ __global__ void k_adj_ef(int n_tets, const int *__restrict__ con, const double *
         const double u = phi[con[4 * e + a]];
         for (int d = 0; d < 3; d++) f[d] = __dsub_rn(f[d], __dmul_rn(nx[12 * e + 3 * a + d], u));
     }
-    for (int d = 0; d < 3; d++) ef[3 * e + d] = f[d];
+    for (int d = 0; d < 3; d++) ef[4 * e + d] = f[d];
+    ef[4 * e + 3] = tets[e].volume;
 }
 
 __global__ void k_adj_wall(int n_tets, const TetRec *__restrict__ tets, const unsigned char *__restrict__ wall_node,
@@ -254,6 +261,7 @@ __device__ __forceinline__ void add_to_tet(bool on, int cell, double (&w)[3], do
     }
 }
 
+template <bool EXACT_CMP>
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_forward(AdjArgs a, double *den) {
     __shared__ double sh[ADJ_THREADS / 32];
     __shared__ unsigned ended[4];
@@ -269,8 +277,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_forward(AdjArgs a, double *
             const int k0 = a.first[p];
             for (int k = k0; k < a.K; k++) {
                 if (k > k0 && k % a.C == 0) store_ck(a, k / a.C - 1, p, s);
-                kick_drift(s, a.ef, a.qm, a.dt);
-                kind = move_cell(a, s, k, p, lc);
+                const double vol = kick_drift(s, a.ef, a.qm, a.dt);
+                kind = move_cell<EXACT_CMP>(a, s, k, p, vol);
                 if (kind != KIND_ALIVE) {
                     ek = k;
                     break;
@@ -282,7 +290,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_forward(AdjArgs a, double *
                 flux += __dmul_rn(a.spwt, __dmul_rn(0.5 * a.mass, v2));
             } else if (kind == KIND_LIMIT) {
                 atomicOr(a.flags, FLAG_WALK_LIMIT);
-            } else if (kind == KIND_ALIVE && a.pinned) {
+            } else if (kind == KIND_ALIVE) {
                 lambdas_fp64(a.tets + s.cell, s.x, s.y, s.z, lc);
             }
             if (kind == KIND_ALIVE) cell = s.cell;
@@ -310,7 +318,8 @@ __global__ void k_adj_normalise(int n_nodes, const double *__restrict__ den, con
     if (i < n_nodes) out[i] = __dmul_rn(den[i], __ddiv_rn(spwt, vol[i]));
 }
 
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_reverse(AdjArgs a, const double *__restrict__ gbar,
+template <bool EXACT_CMP>
+__global__ void __launch_bounds__(ADJ_THREADS, 4) k_adj_reverse(AdjArgs a, const double *__restrict__ gbar,
                                                               const double *__restrict__ vol, double fbar,
                                                               double *ebar) {
     __shared__ double sh[ADJ_THREADS / 32];
@@ -342,10 +351,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_reverse(AdjArgs a, const do
             const int ke = s0 + a.C - 1 < last ? s0 + a.C - 1 : last;  // below kb: no step of this segment
             if (on && kb <= ke) {
                 Slot s = kb == k0 ? start_slot(a, p) : load_ck(a, j - 1, p);
-                double lc[4];
                 for (int k = kb; k <= ke; k++) {
                     cs[k - s0] = s.cell;
-                    kick_drift(s, a.ef, a.qm, a.dt);
+                    const double v0 = kick_drift(s, a.ef, a.qm, a.dt);
                     if (k == last) {
                         if (kind == KIND_WALL) {
                             const double c = fbar * a.spwt * a.mass;
@@ -354,7 +362,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_reverse(AdjArgs a, const do
                             vb[2] = c * s.vz;
                         }
                     } else if (k < ke) {
-                        move_cell(a, s, k, p, lc);
+                        move_cell<EXACT_CMP>(a, s, k, p, v0);
                     }
                 }
             }
@@ -403,6 +411,7 @@ __global__ void k_adj_phibar(int n_tets, const int *__restrict__ con, const doub
 }
 
 // Tangent: d(den raw), d(flux) along (dphi -> def, dvd), replaying the tape's cells.
+template <bool EXACT_CMP>
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_tangent(AdjArgs a, const double *__restrict__ def, double dvd,
                                                               double *dden) {
     __shared__ double sh[ADJ_THREADS / 32];
@@ -416,20 +425,21 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_tangent(AdjArgs a, const do
             const int k0 = a.first[p];
             double dx[3] = {0, 0, 0}, dv[3] = {0, 0, 0};
             if (a.inj[p]) {
-                const double *de = def + 3 * s.cell;
+                double de[4];
+                load32(def + 4 * (long long)s.cell, de);
                 const double dir[3] = {a.dir0, a.dir1, a.dir2};
                 for (int d = 0; d < 3; d++) dv[d] = dir[d] * dvd - a.qm * de[d] * (0.5 * a.dt);
             }
             int kind = KIND_ALIVE;
-            double lc[4];
             for (int k = k0; k < a.K; k++) {
-                const double *de = def + 3 * s.cell;
+                double de[4];
+                load32(def + 4 * (long long)s.cell, de);
                 for (int d = 0; d < 3; d++) {
                     dv[d] += a.qm * de[d] * a.dt;
                     dx[d] += dv[d] * a.dt;
                 }
-                kick_drift(s, a.ef, a.qm, a.dt);
-                kind = move_cell(a, s, k, p, lc);
+                const double vol = kick_drift(s, a.ef, a.qm, a.dt);
+                kind = move_cell<EXACT_CMP>(a, s, k, p, vol);
                 if (kind != KIND_ALIVE) break;
             }
             if (kind == KIND_WALL) {
@@ -518,7 +528,9 @@ static AdjArgs args_of(mp_ctx *ctx, AdjState *s, bool pinned, bool record) {
 
 static int grid_of(mp_ctx *ctx, long long n) {
     long long g = (n + ADJ_THREADS - 1) / ADJ_THREADS;
-    long long cap = (long long)ctx->sm_count * 8;
+    // many short blocks: a block lasts as long as its slots live and hop (8 an SM: 1.18 ms
+    // for a forward and reverse of 1M ions, 64: 1.00)
+    long long cap = (long long)ctx->sm_count * 64;
     return (int)std::max(1ll, std::min(g, cap));
 }
 
@@ -595,8 +607,8 @@ int mp_adjoint_setup(mp_ctx *ctx, int32_t steps, int32_t checkpoint_every, doubl
     } else {
         s->nx = ctx->nx;
     }
-    MP_CUDA(ctx, cudaMalloc(&s->ef, sizeof(double) * 3 * nt));
-    MP_CUDA(ctx, cudaMalloc(&s->def, sizeof(double) * 3 * nt));
+    MP_CUDA(ctx, cudaMalloc(&s->ef, sizeof(double) * 4 * nt));
+    MP_CUDA(ctx, cudaMalloc(&s->def, sizeof(double) * 4 * nt));
     MP_CUDA(ctx, cudaMalloc(&s->wall, nt));
     MP_CUDA(ctx, cudaMalloc(&s->nodes_a, sizeof(double) * nn));
     MP_CUDA(ctx, cudaMalloc(&s->nodes_b, sizeof(double) * nn));
@@ -659,7 +671,7 @@ int mp_adjoint_forward(mp_ctx *ctx, const double *phi, double v_drift, int mode,
     const int nt = ctx->n_tets, nn = ctx->n_nodes;
     cudaEventRecord(ctx->t0.a, ctx->stream);
     MP_CUDA(ctx, cudaMemcpyAsync(s->nodes_b, phi, sizeof(double) * nn, cudaMemcpyDefault, ctx->stream));
-    k_adj_ef<<<(nt + 255) / 256, 256, 0, ctx->stream>>>(nt, ctx->con, s->nx, s->nodes_b, s->ef), ++ctx->launches;
+    k_adj_ef<<<(nt + 255) / 256, 256, 0, ctx->stream>>>(nt, ctx->con, s->nx, s->nodes_b, ctx->tets, s->ef), ++ctx->launches;
     MP_CUDA(ctx, cudaMemsetAsync(s->nodes_a, 0, sizeof(double) * nn, ctx->stream));
     MP_CUDA(ctx, cudaMemsetAsync(s->scal, 0, sizeof(double) * 8, ctx->stream));
     s->vd = v_drift;
@@ -667,7 +679,9 @@ int mp_adjoint_forward(mp_ctx *ctx, const double *phi, double v_drift, int mode,
     const bool record = s->record && !pinned;
     AdjArgs a = args_of(ctx, s, pinned, record);
     if (s->n > 0)
-        k_adj_forward<<<grid_of(ctx, s->n), ADJ_THREADS, 0, ctx->stream>>>(a, s->nodes_a), ++ctx->launches;
+        (ctx->small_tets ? k_adj_forward<true> : k_adj_forward<false>)<<<grid_of(ctx, s->n), ADJ_THREADS, 0, ctx->stream>>>(
+            a, s->nodes_a),
+            ++ctx->launches;
     k_adj_normalise<<<(nn + 255) / 256, 256, 0, ctx->stream>>>(nn, s->nodes_a, ctx->node_volume, s->spwt,
                                                                s->nodes_b), ++ctx->launches;
     MP_CUDA(ctx, cudaGetLastError());
@@ -723,8 +737,9 @@ int mp_adjoint_backward(mp_ctx *ctx, const double *den_bar, double flux_bar, dou
     MP_CUDA(ctx, cudaMemsetAsync(s->scal + 1, 0, sizeof(double), ctx->stream));
     AdjArgs a = args_of(ctx, s, s->mode == MP_ADJ_PINNED, false);
     if (s->n > 0)
-        k_adj_reverse<<<grid_of(ctx, s->n), ADJ_THREADS, 0, ctx->stream>>>(a, s->nodes_a, ctx->node_volume, flux_bar,
-                                                                          s->def), ++ctx->launches;
+        (ctx->small_tets ? k_adj_reverse<true> : k_adj_reverse<false>)<<<grid_of(ctx, s->n), ADJ_THREADS, 0, ctx->stream>>>(
+            a, s->nodes_a, ctx->node_volume, flux_bar, s->def),
+            ++ctx->launches;
     k_adj_phibar<<<(nt + 255) / 256, 256, 0, ctx->stream>>>(nt, ctx->con, s->nx, s->def, s->nodes_b),
         ++ctx->launches;
     MP_CUDA(ctx, cudaGetLastError());
@@ -742,16 +757,17 @@ int mp_adjoint_tangent(mp_ctx *ctx, const double *dphi, double dv_drift, double 
     const int nt = ctx->n_tets, nn = ctx->n_nodes;
     if (dphi) {
         MP_CUDA(ctx, cudaMemcpyAsync(s->nodes_b, dphi, sizeof(double) * nn, cudaMemcpyDefault, ctx->stream));
-        k_adj_ef<<<(nt + 255) / 256, 256, 0, ctx->stream>>>(nt, ctx->con, s->nx, s->nodes_b, s->def),
+        k_adj_ef<<<(nt + 255) / 256, 256, 0, ctx->stream>>>(nt, ctx->con, s->nx, s->nodes_b, ctx->tets, s->def),
             ++ctx->launches;
     } else {
-        MP_CUDA(ctx, cudaMemsetAsync(s->def, 0, sizeof(double) * 3 * nt, ctx->stream));
+        MP_CUDA(ctx, cudaMemsetAsync(s->def, 0, sizeof(double) * 4 * nt, ctx->stream));
     }
     MP_CUDA(ctx, cudaMemsetAsync(s->nodes_a, 0, sizeof(double) * nn, ctx->stream));
     MP_CUDA(ctx, cudaMemsetAsync(s->scal + 2, 0, sizeof(double), ctx->stream));
     AdjArgs a = args_of(ctx, s, s->mode == MP_ADJ_PINNED, false);
     if (s->n > 0)
-        k_adj_tangent<<<grid_of(ctx, s->n), ADJ_THREADS, 0, ctx->stream>>>(a, s->def, dv_drift, s->nodes_a),
+        (ctx->small_tets ? k_adj_tangent<true> : k_adj_tangent<false>)<<<grid_of(ctx, s->n), ADJ_THREADS, 0, ctx->stream>>>(
+            a, s->def, dv_drift, s->nodes_a),
             ++ctx->launches;
     k_adj_normalise<<<(nn + 255) / 256, 256, 0, ctx->stream>>>(nn, s->nodes_a, ctx->node_volume, s->spwt,
                                                                s->nodes_b), ++ctx->launches;

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(PUSH_THREADS, 4) k_push_fp64(PushF64Args a) {
             x = __dadd_rn(x, __dmul_rn(vx, a.dt));
             y = __dadd_rn(y, __dmul_rn(vy, a.dt));
             z = __dadd_rn(z, __dmul_rn(vz, a.dt));
-            int w = walk_fp64<EXACT_CMP>(a.tets, cell, x, y, z, lc, a.walk_limit, hops);
+            int w = walk_fp64<EXACT_CMP>(a.tets, cell, x, y, z, ef[3], lc, a.walk_limit, hops);
             if (w == 1) {
                 state = 1;
                 const int4 c4 = __ldg(reinterpret_cast<const int4 *>(a.tets[cell].con));

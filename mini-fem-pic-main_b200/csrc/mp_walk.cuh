@@ -70,15 +70,15 @@ __device__ __forceinline__ void lambdas_fp64(const TetRec *__restrict__ t, doubl
 // and NaN compares false either way.  An inside particle's weights for the
 // scatter are then q*RN(1/V) (within 2 ulp of lambda).  A particle outside its
 // tet needs the exact lambdas for the hop (first minimum, strict <), so those
-// are divided.
+// are divided.  vol: the volume of the tet the walk starts in.
 template <bool EXACT_CMP = false>
 __device__ __forceinline__ int walk_fp64(const TetRec *__restrict__ tets, int &cell, double x, double y, double z,
-                                         double lc[4], int limit, int &hops, int *exit_face = nullptr) {
+                                         double vol, double lc[4], int limit, int &hops,
+                                         int *exit_face = nullptr) {
     for (;;) {
         const TetRec *t = tets + cell;
         double q[4];
         numerators_fp64(t, x, y, z, q);
-        const double vol = __ldg(&t->volume);
         if (EXACT_CMP) {
             bool inside = true;
 #pragma unroll
@@ -116,6 +116,7 @@ __device__ __forceinline__ int walk_fp64(const TetRec *__restrict__ tets, int &c
         }
         if (hops >= limit) return -1;
         cell = nb;
+        vol = __ldg(&tets[nb].volume);
         hops++;
     }
 }
