@@ -439,6 +439,18 @@ static int grid_for(mp_ctx *ctx, const void *kernel, int threads, size_t smem) {
     return per_sm * ctx->sm_count;
 }
 
+// CTAs of a push: one wave of resident ones, or 3 to 8 waves of at least 4,096
+// particles a CTA.  A CTA's block of particles takes its time by their hops and
+// the mesh's band they lie in, and one wave ends with its slowest CTA: 48M ions
+// FP64 1.97 -> 1.51 ms, mixed 1.24 -> 1.00, 16M 665 -> 551 and 420 -> 375 us.  Two
+// waves, or smaller blocks, cost the L1's reuse more than they balance (mixed, 4M
+// ions: 97 us in one wave, 113 in two; FP64, 2M: 77, 80 and in four 87).
+static long long push_ctas(long long blocks, long long resident, long long n) {
+    if (blocks < resident) return blocks;
+    const long long waves = std::min(8ll, n / (4096 * resident));
+    return resident * (waves < 3 ? 1 : waves);
+}
+
 int launch_push(mp_ctx *ctx, double q_over_m, double dt) {
     long long blocks = (ctx->n_host + PUSH_THREADS - 1) / PUSH_THREADS;
     if (blocks < 1) blocks = 1;
@@ -458,7 +470,7 @@ int launch_push(mp_ctx *ctx, double q_over_m, double dt) {
         // division-free inside test when every tet volume is below 1 (see walk_fp64)
         auto kern = ctx->small_tets ? k_push_fp64<true> : k_push_fp64<false>;
         if (!ctx->push_grid[0]) ctx->push_grid[0] = grid_for(ctx, (const void *)kern, PUSH_THREADS, 0);
-        long long g = blocks < ctx->push_grid[0] ? blocks : ctx->push_grid[0];
+        const long long g = push_ctas(blocks, ctx->push_grid[0], ctx->n_host);
         cudaEventRecord(ctx->tp.a, ctx->stream);
         kern<<<(unsigned)g, PUSH_THREADS, 0, ctx->stream>>>(a), ++ctx->launches;
         cudaEventRecord(ctx->tp.b, ctx->stream);
@@ -478,7 +490,7 @@ int launch_push(mp_ctx *ctx, double q_over_m, double dt) {
         a.fixed = ctx->scatter_mode == MP_SCATTER_FIXED64;
         a.track_ids = ctx->track_ids;
         if (!ctx->push_grid[1]) ctx->push_grid[1] = grid_for(ctx, (const void *)k_push_mixed, PUSH_THREADS, 0);
-        long long g = blocks < ctx->push_grid[1] ? blocks : ctx->push_grid[1];
+        const long long g = push_ctas(blocks, ctx->push_grid[1], ctx->n_host);
         cudaEventRecord(ctx->tp.a, ctx->stream);
         k_push_mixed<<<(unsigned)g, PUSH_THREADS, 0, ctx->stream>>>(a), ++ctx->launches;
         cudaEventRecord(ctx->tp.b, ctx->stream);
