@@ -50,7 +50,7 @@ constexpr double WEIGHT = 0.3;              // of each level's correction
 constexpr double MASS = 0.35;               // sum of phi^2 over sum of phi, about, of a function of any level
 constexpr int HALO_REGS = 4, OWN_REGS = 4, TASK_REGS = 4;  // a thread's halo rows, functions and runs, at most
 constexpr int RUN = 8;                      // shares added by one thread
-constexpr size_t SMEM_MAX = 227 * 1024;
+constexpr int SMEM_MAX = 227 * 1024 - 2048; // dynamic shared memory of a plan, beside the kernel's static one
 
 enum Status : unsigned { NOT_SPD = 1, TIMEOUT = 2, MAX_IT = 4 };
 
@@ -1184,7 +1184,7 @@ static int make_plan(mp_ctx *ctx, Plan *p, const std::vector<long long> &rowp, c
     p->smem = sizeof(Place) * a.nl_max + sizeof(double) * (2 * (size_t)a.nl_max + 3 * (size_t)a.need_max + a.u_max + 4 * WARPS + 4) +
               sizeof(unsigned) * a.need_max + sizeof(unsigned short) * (a.need_max + 1 + a.nc_max + 1 + (a.need_max + a.nc_max & 1)) +
               sizeof(int) * (2 * a.own_max + a.task_max + a.halo_max + a.nr_max / 32 + 2);
-    const size_t most = SMEM_MAX - 2048;    // beside the kernel's static shared memory
+    const size_t most = SMEM_MAX;
     if (p->smem > most || a.nfn - a.lev[a.full].off - a.lev[a.full].n > FULL_MAX) return MP_OK;
     int columns = 0;
     for (int b = 0; b < nb; b++) columns = std::max(columns, (slice_ptr[slice_off[b + 1]] - slice_ptr[slice_off[b]]) / 32);
@@ -1268,7 +1268,9 @@ int cg_levels_setup(mp_ctx *ctx, const std::vector<long long> &rowp, const std::
 
 template <int RPT>
 static cudaError_t launch(const Plan *p, Args a, cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(k_cg_levels<RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
+    // the attribute is the function's, shared by all contexts: what any plan may need, so that
+    // one thread's launch never finds another's smaller limit
+    cudaError_t e = cudaFuncSetAttribute(k_cg_levels<RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
     if (e != cudaSuccess) return e;
     void *args[] = {&a};
     return cudaLaunchCooperativeKernel((const void *)k_cg_levels<RPT>, dim3(a.nb), dim3(THREADS), args, p->smem, stream);
