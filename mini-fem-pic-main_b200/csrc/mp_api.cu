@@ -161,6 +161,14 @@ int ensure_dstage(mp_ctx *ctx, size_t bytes) {
     return MP_OK;
 }
 
+// Device memory, if there is any: false, and no error left, if there is not.
+bool device_room(void **p, size_t bytes) {
+    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    *p = nullptr;
+    return false;
+}
+
 // Waits for the stream and turns the host's copy of the counters, which the
 // last kernel or copy in the stream wrote, into counts and a status.
 static int read_counters(mp_ctx *ctx) {

@@ -833,14 +833,6 @@ void bisect(const float *pos, int *idx, int first, int last, int parts, int part
     if (other.joinable()) other.join();
 }
 
-// Device memory, if there is any: a plan without it is unusable, no error.
-bool room(void **p, size_t bytes) {
-    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
-    cudaGetLastError();
-    *p = nullptr;
-    return false;
-}
-
 Plan *plan_of(mp_ctx *ctx) { return static_cast<Plan *>(ctx->cg_levels); }
 
 }  // namespace
@@ -1204,7 +1196,7 @@ static int make_plan(mp_ctx *ctx, Plan *p, const std::vector<long long> &rowp, c
 #define X(v) const size_t o_##v = take(v.size() * sizeof(v[0]));
     CG_ARRAYS(X)
 #undef X
-    if (!room((void **)&p->blob, off)) return MP_OK;
+    if (!device_room((void **)&p->blob, off)) return MP_OK;  // unusable, no error
     unsigned char *base = static_cast<unsigned char *>(p->blob);
 #define X(v) \
     if (!v.empty()) MP_CUDA(ctx, cudaMemcpy(base + o_##v, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
@@ -1225,7 +1217,7 @@ static int make_plan(mp_ctx *ctx, Plan *p, const std::vector<long long> &rowp, c
     const size_t o_val = take(8 * total), o_kd = take(8 * (size_t)n), o_e = take(8 * 36 * (size_t)ncells),
                  o_dk = take(8 * (size_t)a.nfn), o_pub = take(16 * (size_t)n), o_share = take(16 * (size_t)a.shares),
                  o_sums = take(8 * 8 * (size_t)nb), o_flag = take(4);
-    if (!room((void **)&p->val, off)) return MP_OK;
+    if (!device_room((void **)&p->val, off)) return MP_OK;
     base = reinterpret_cast<unsigned char *>(p->val);
     auto at = [&](size_t o) { return reinterpret_cast<double *>(base + o); };
     p->kd = at(o_kd);

@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "mp_alloc.h"
 #include "mp_internal.h"
 
 namespace mp {
@@ -343,10 +344,12 @@ int gs_prepare(mp_ctx *ctx, bool *usable) {
             off[k] = end;
             end = (end + bytes[k] + 255) & ~size_t(255);
         }
-        MP_CUDA(ctx, cudaMalloc(&s->blob, end));
+        if (!allocate_all({{&s->blob, end}, {(void **)&s->out, sizeof(double) * 4}}, device_room, cudaFree)) {
+            gs_free(ctx);  // the dense sweeps take the call, and the next one asks again
+            return MP_OK;
+        }
         char *base = static_cast<char *>(s->blob);
         for (int k = 0; k < 8; k++) MP_CUDA(ctx, cudaMemcpy(base + off[k], src[k], bytes[k], cudaMemcpyHostToDevice));
-        MP_CUDA(ctx, cudaMalloc(&s->out, sizeof(double) * 4));
         MP_CUDA(ctx, cudaHostAlloc(&s->out_host, sizeof(double) * 4, 0));
         const int most = (int)sizeof(double) * 1024 * GS_MAX_CLUSTER;
         MP_CUDA(ctx, cudaFuncSetAttribute(k_gs_cluster<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));

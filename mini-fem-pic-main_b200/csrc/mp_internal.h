@@ -251,6 +251,7 @@ int cuda_fail(mp_ctx *ctx, cudaError_t e, const char *what);
 
 // Kernels' host launchers (push / field / solver translation units).
 int ensure_dstage(mp_ctx *ctx, size_t bytes);
+bool device_room(void **p, size_t bytes);
 int launch_push(mp_ctx *ctx, double q_over_m, double dt);
 int launch_normalise(mp_ctx *ctx, double spwt);
 int launch_append(mp_ctx *ctx, long long n, const double *pos_soa, const double *vel_soa, const int *cell,

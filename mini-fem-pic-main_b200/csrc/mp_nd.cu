@@ -27,6 +27,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "mp_alloc.h"
 #include "mp_internal.h"
 #include "mp_nd.h"
 
@@ -1052,8 +1053,9 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_nd_solve(SolveArgs a) {
 }
 
 struct NdState {
-    bool usable = false;               // the plan exists and is the faster way
-    NdPlan plan;                       // (its host lists are dropped once on the device)
+    bool planned = false;              // the plan exists
+    bool usable = false;               // and is on the device, with the factor's memory
+    NdPlan plan;                       // (its long host lists are dropped once on the device)
     void *blob = nullptr;              // the plan's arrays
     const NdTask *task = nullptr;
     const NdItem *item = nullptr;
@@ -1072,12 +1074,19 @@ NdState *state_of(mp_ctx *ctx) { return static_cast<NdState *>(ctx->nd); }
 
 }  // namespace
 
+static void nd_release(NdState *s) {
+    void **p[] = {&s->blob, (void **)&s->tile, (void **)&s->zd, (void **)&s->x, (void **)&s->flag, (void **)&s->ctl};
+    for (void **q : p) {
+        if (*q) cudaFree(*q);
+        *q = nullptr;
+    }
+    s->usable = false;
+}
+
 void nd_free(mp_ctx *ctx) {
     NdState *s = state_of(ctx);
     if (!s) return;
-    void *p[] = {s->blob, s->tile, s->zd, s->x, s->flag, s->ctl};
-    for (void *q : p)
-        if (q) cudaFree(q);
+    nd_release(s);
     delete s;
     ctx->nd = nullptr;
 }
@@ -1093,19 +1102,71 @@ static bool nd_faster(long long products, int chain, int n, int sms, bool mixed)
     return nd < dense;
 }
 
-// Builds the plan on the first direct solve after mp_fe_setup.  *usable: the
-// sparse factorization applies (K has the mesh's pattern and is symmetric) and
-// is expected to be faster than the dense one.
+// Puts the plan on the device, with the factor's memory (the largest part first).
+// Where that cannot be had, the state stays unusable and takes none.
+static int nd_place(mp_ctx *ctx, NdState *s) {
+    NdPlan &p = s->plan;
+    size_t off = 0;
+    auto place = [&](size_t bytes) {
+        const size_t o = off;
+        off = (off + bytes + 255) & ~size_t(255);
+        return o;
+    };
+#define ND_ARRAYS(X) X(task) X(item) X(perm) X(ent_src) X(ent_at) X(tile_ptr) X(tile_row) X(tile_col) X(row_ptr) X(row_tile)
+    std::vector<unsigned char> host;
+#define X(a) const size_t o_##a = place(p.a.size() * sizeof(p.a[0]));
+    ND_ARRAYS(X)
+#undef X
+    host.resize(off + 256);
+#define X(a) if (!p.a.empty()) std::memcpy(host.data() + o_##a, p.a.data(), p.a.size() * sizeof(p.a[0]));
+    ND_ARRAYS(X)
+#undef X
+    s->words = (size_t)p.ntile + p.nscratch;
+    if (!allocate_all({{(void **)&s->tile, sizeof(double) * s->words * TT},
+                       {&s->blob, host.size()},
+                       {(void **)&s->zd, sizeof(double) * (size_t)(p.ncol + p.nscratch) * ZD},
+                       {(void **)&s->x, sizeof(double) * (size_t)p.ncol * T},
+                       {(void **)&s->flag, sizeof(unsigned) * s->words},
+                       {(void **)&s->ctl, sizeof(unsigned) * 8}},
+                      device_room, cudaFree))
+        return MP_OK;
+    MP_CUDA(ctx, cudaMemcpy(s->blob, host.data(), host.size(), cudaMemcpyHostToDevice));
+#define X(a) s->a = reinterpret_cast<decltype(s->a)>(static_cast<unsigned char *>(s->blob) + o_##a);
+    ND_ARRAYS(X)
+#undef X
+#undef ND_ARRAYS
+    s->ntask = (int)p.task.size();
+    // the blocks above an inverse's diagonal stay zero
+    MP_CUDA(ctx, cudaMemsetAsync(s->tile, 0, sizeof(double) * (size_t)p.ntile * TT, ctx->stream));
+    MP_CUDA(ctx, cudaMemsetAsync(s->flag, 0, sizeof(unsigned) * s->words, ctx->stream));
+    MP_CUDA(ctx, cudaFuncSetAttribute(k_nd_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
+    MP_CUDA(ctx, cudaFuncSetAttribute(k_nd_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(SolveSmem)));
+    MP_CUDA(ctx, cudaFuncSetAttribute(k_nd_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(SolveSmem)));
+    p.task.clear();
+    p.task.shrink_to_fit();
+    p.item.clear();
+    p.item.shrink_to_fit();
+    s->epoch = 0;
+    s->usable = true;
+    return MP_OK;
+}
+
+// Builds the plan on the first direct solve after mp_fe_setup, and places it when
+// it is first the faster way.  *usable: the sparse factorization applies (K has the
+// mesh's pattern and is symmetric), is expected to be faster than the dense one
+// and has its memory; a device too full for it is asked again by the next call.
 int nd_prepare(mp_ctx *ctx, bool mixed, bool *usable) {
     *usable = false;
     NdState *s = state_of(ctx);
+    int rc;
     if (!s) {
         s = new NdState();
         ctx->nd = s;
         const int n = ctx->neq;
         bool fits = false;
-        int rc = fe_pattern_fits(ctx, &fits);
-        if (rc) return rc;
+        if ((rc = fe_pattern_fits(ctx, &fits))) return rc;
         if (fits && !ctx->csr_ptr.empty()) {
             std::vector<double> pos(3 * (size_t)n, 0.0), npos(3 * (size_t)ctx->n_nodes);
             std::vector<int> ID(ctx->n_nodes);
@@ -1116,53 +1177,15 @@ int nd_prepare(mp_ctx *ctx, bool mixed, bool *usable) {
                     for (int d = 0; d < 3; d++) pos[3 * (size_t)ID[k] + d] = npos[3 * (size_t)k + d];
             const double blocks = n / 64.0 + 1;
             const long long most = (long long)(blocks * blocks * blocks / 6 + 100);
-            s->usable = nd_build_plan(n, ctx->csr_ptr, ctx->csr_col, ctx->csr_slot, pos, most, s->plan);
-        }
-        if (s->usable) {
-            NdPlan &p = s->plan;
-            size_t off = 0;
-            auto place = [&](size_t bytes) {
-                const size_t o = off;
-                off = (off + bytes + 255) & ~size_t(255);
-                return o;
-            };
-#define ND_ARRAYS(X) X(task) X(item) X(perm) X(ent_src) X(ent_at) X(tile_ptr) X(tile_row) X(tile_col) X(row_ptr) X(row_tile)
-            std::vector<unsigned char> host;
-#define X(a) const size_t o_##a = place(p.a.size() * sizeof(p.a[0]));
-            ND_ARRAYS(X)
-#undef X
-            host.resize(off + 256);
-#define X(a) if (!p.a.empty()) std::memcpy(host.data() + o_##a, p.a.data(), p.a.size() * sizeof(p.a[0]));
-            ND_ARRAYS(X)
-#undef X
-            MP_CUDA(ctx, cudaMalloc(&s->blob, host.size()));
-            MP_CUDA(ctx, cudaMemcpy(s->blob, host.data(), host.size(), cudaMemcpyHostToDevice));
-#define X(a) s->a = reinterpret_cast<decltype(s->a)>(static_cast<unsigned char *>(s->blob) + o_##a);
-            ND_ARRAYS(X)
-#undef X
-#undef ND_ARRAYS
-            s->ntask = (int)p.task.size();
-            MP_CUDA(ctx, cudaMalloc(&s->tile, sizeof(double) * (size_t)(p.ntile + p.nscratch) * TT));
-            MP_CUDA(ctx, cudaMalloc(&s->zd, sizeof(double) * (size_t)(p.ncol + p.nscratch) * ZD));
-            MP_CUDA(ctx, cudaMalloc(&s->x, sizeof(double) * (size_t)p.ncol * T));
-            // the blocks above an inverse's diagonal stay zero
-            MP_CUDA(ctx, cudaMemsetAsync(s->tile, 0, sizeof(double) * (size_t)p.ntile * TT, ctx->stream));
-            s->words = (size_t)p.ntile + p.nscratch;
-            MP_CUDA(ctx, cudaMalloc(&s->flag, sizeof(unsigned) * s->words));
-            MP_CUDA(ctx, cudaMemsetAsync(s->flag, 0, sizeof(unsigned) * s->words, ctx->stream));
-            MP_CUDA(ctx, cudaMalloc(&s->ctl, sizeof(unsigned) * 8));
-            MP_CUDA(ctx, cudaFuncSetAttribute(k_nd_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
-            MP_CUDA(ctx, cudaFuncSetAttribute(k_nd_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)sizeof(SolveSmem)));
-            MP_CUDA(ctx, cudaFuncSetAttribute(k_nd_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)sizeof(SolveSmem)));
-            s->plan.task.clear();
-            s->plan.task.shrink_to_fit();
-            s->plan.item.clear();
-            s->plan.item.shrink_to_fit();
+            s->planned = nd_build_plan(n, ctx->csr_ptr, ctx->csr_col, ctx->csr_slot, pos, most, s->plan);
         }
     }
-    *usable = s->usable && nd_faster(s->plan.products, s->plan.chain, ctx->neq, ctx->sm_count, mixed);
+    if (!s->planned || !nd_faster(s->plan.products, s->plan.chain, ctx->neq, ctx->sm_count, mixed)) return MP_OK;
+    if (!s->usable && (rc = nd_place(ctx, s))) {
+        nd_release(s);
+        return rc;
+    }
+    *usable = s->usable;
     return MP_OK;
 }
 

@@ -592,16 +592,13 @@ int fe_pattern_fits(mp_ctx *ctx, bool *fits) {
     if (ctx->k_given && ctx->k_fits < 0) {
         const int n = ctx->neq;
         const long long ld = (n + 31) & ~31ll;
-        unsigned long long *cnt = nullptr, h[3] = {0, 0, 0};
-        MP_CUDA(ctx, cudaMalloc(&cnt, sizeof(h)));
-        cudaMemsetAsync(cnt, 0, sizeof(h), ctx->stream);
+        unsigned long long *cnt = reinterpret_cast<unsigned long long *>(ctx->scal), h[3] = {0, 0, 0};
+        MP_CUDA(ctx, cudaMemsetAsync(cnt, 0, sizeof(h), ctx->stream));
         k_check_dense<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(n, ld, ctx->K, cnt), ++ctx->launches;
         k_count_sparse<<<(n + 255) / 256, 256, 0, ctx->stream>>>(n, ctx->sp_len, ctx->sp_ptr, ctx->sp_val, cnt),
             ++ctx->launches;
-        cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
-        cudaError_t e = cudaStreamSynchronize(ctx->stream);
-        cudaFree(cnt);
-        MP_CUDA(ctx, e);
+        MP_CUDA(ctx, cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+        MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         ctx->k_fits = h[0] == 0 && h[1] == h[2];
     }
     *fits = !ctx->k_given || ctx->k_fits > 0;
