@@ -1,6 +1,5 @@
-// Device memory that is taken when it is first needed: all of it or none, so
-// that a call which meets a full device leaves a state that the next call can
-// use.
+// Device memory that is taken when it is first needed, in a way that leaves a
+// state the next call can use where a call meets a full device.
 #pragma once
 
 #include <cstddef>
@@ -28,6 +27,21 @@ bool allocate_all(std::initializer_list<Block> blocks, Alloc alloc, Release rele
         }
         return false;
     }
+    return true;
+}
+
+// Makes p, of len elements, hold at least `need`: by a new array of `size`, the old
+// contents lost.  Where that cannot be had: p null, len 0 and false.
+template <typename T, typename Alloc, typename Release>
+bool grow(T *&p, long long &len, long long need, long long size, Alloc alloc, Release release) {
+    if (p && len >= need) return true;
+    if (p) release(p);
+    p = nullptr;
+    len = 0;
+    void *q = nullptr;
+    if (!alloc(&q, sizeof(T) * (size_t)size)) return false;
+    p = static_cast<T *>(q);
+    len = size;
     return true;
 }
 

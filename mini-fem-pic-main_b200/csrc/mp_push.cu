@@ -12,6 +12,7 @@
 // Observable results (particle list, density) are those of a per-step removal.
 #include <algorithm>
 
+#include "mp_alloc.h"
 #include "mp_internal.h"
 #include "mp_walk.cuh"
 #include "mp_warp.cuh"
@@ -560,12 +561,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int m, int *v, int *part,
 
 static int launch_scan(mp_ctx *ctx, int m, int *v, bool set_counts) {
     const long long blocks = (m + SCAN_TILE - 1) / SCAN_TILE;
-    if (ctx->scan_part_len < blocks) {
-        if (ctx->scan_part) cudaFree(ctx->scan_part);
-        ctx->scan_part = nullptr;
-        MP_CUDA(ctx, cudaMalloc(&ctx->scan_part, sizeof(int) * 2 * blocks));
-        ctx->scan_part_len = 2 * blocks;
-    }
+    if (!grow(ctx->scan_part, ctx->scan_part_len, blocks, 2 * blocks, device_room, cudaFree))
+        return cuda_fail(ctx, cudaErrorMemoryAllocation, "cudaMalloc(scan_part)");
     k_scan<<<(unsigned)blocks, SCAN_THREADS, 0, ctx->stream>>>(m, v, ctx->scan_part, ctx->counters + C_TICKET,
                                                               set_counts ? ctx->counters : nullptr), ++ctx->launches;
     MP_CUDA(ctx, cudaGetLastError());

@@ -1,6 +1,6 @@
-"""Host: memory taken all or none (csrc/mp_alloc.h), with an allocator that fails
-at each of its calls in turn: no pointer is left set, nothing is left allocated
-and nothing is freed twice."""
+"""Host: memory taken all or none, and arrays that grow (csrc/mp_alloc.h), with an
+allocator that fails at each of its calls in turn: no pointer and no length is
+left set, nothing is left allocated and nothing is freed twice."""
 from __future__ import annotations
 
 import os
@@ -38,6 +38,16 @@ int main() {
         if (ok != (fail_at == 3)) return 2;
         if (ok ? live.size() != 3 || !a || !b || !c : !live.empty() || a || b || c) return 3;
     }
+    for (void *p : std::set<void *>(live)) give(p);
+    // an array grows, fails to, and is asked for less than it held before
+    int *p = nullptr;
+    long long len = 0;
+    calls = 0;
+    fail_at = 1;
+    if (!mp::grow(p, len, 10, 20, take, give) || len != 20 || live.count(p) != 1) return 4;
+    if (!mp::grow(p, len, 20, 40, take, give) || len != 20 || calls != 1) return 5;
+    if (mp::grow(p, len, 21, 42, take, give) || p || len || !live.empty()) return 6;
+    if (!mp::grow(p, len, 5, 10, take, give) || len != 10 || live.size() != 1) return 7;
     return 0;
 }
 """
