@@ -27,7 +27,6 @@
 #include <cmath>
 #include <cstring>
 #include <exception>
-#include <system_error>
 #include <thread>
 
 #include "mp_internal.h"
@@ -787,7 +786,7 @@ void in_parallel(int n, F work) {
     for (int k = 1; k < th; k++) {
         try {
             pool.emplace_back(part, k);
-        } catch (const std::system_error &) {
+        } catch (const std::exception &) {
             part(k);
         }
     }
@@ -825,7 +824,7 @@ void bisect(const float *pos, int *idx, int first, int last, int parts, int part
     if (fork > 0) {
         try {
             other = std::thread(bisect, pos, idx, first, mid, left, part0, end, fork - 1);
-        } catch (const std::system_error &) {
+        } catch (const std::exception &) {
         }
     }
     if (!other.joinable()) bisect(pos, idx, first, mid, left, part0, end, 0);

@@ -29,6 +29,7 @@
 // and takes 0.50 ms.
 #include <algorithm>
 #include <cmath>
+#include <exception>
 
 #include "mp_alloc.h"
 #include "mp_internal.h"
@@ -239,11 +240,7 @@ void gs_free(mp_ctx *ctx) {
     ctx->gs = nullptr;
 }
 
-// Plans the solve on its first use after mp_fe_setup.  *usable: every row fits
-// a thread and all rows one cluster of at most 8 CTAs, and K has the mesh's
-// pattern.
-int gs_prepare(mp_ctx *ctx, bool *usable) {
-    *usable = false;
+static int gs_plan(mp_ctx *ctx, bool *usable) {
     GsState *s = static_cast<GsState *>(ctx->gs);
     if (!s) {
         s = new GsState();
@@ -345,7 +342,7 @@ int gs_prepare(mp_ctx *ctx, bool *usable) {
             end = (end + bytes[k] + 255) & ~size_t(255);
         }
         if (!allocate_all({{&s->blob, end}, {(void **)&s->out, sizeof(double) * 4}}, device_room, cudaFree)) {
-            gs_free(ctx);  // the dense sweeps take the call, and the next one asks again
+            gs_free(ctx);
             return MP_OK;
         }
         char *base = static_cast<char *>(s->blob);
@@ -371,6 +368,20 @@ int gs_prepare(mp_ctx *ctx, bool *usable) {
     }
     *usable = s->usable;
     return MP_OK;
+}
+
+// Plans the solve on its first use after mp_fe_setup.  *usable: every row fits
+// a thread and all rows one cluster of at most 8 CTAs, and K has the mesh's
+// pattern.  Where the device or the host is too full for the plan, the dense
+// sweeps take the call and the next call asks again.
+int gs_prepare(mp_ctx *ctx, bool *usable) {
+    *usable = false;
+    try {
+        return gs_plan(ctx, usable);
+    } catch (const std::exception &) {
+        gs_free(ctx);
+        return MP_OK;
+    }
 }
 
 // Sweeps J y = G from the current y; FP is J's diagonal term.  *stop: a device word

@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
 
 #include "mp_alloc.h"
 #include "mp_internal.h"
@@ -1153,12 +1154,7 @@ static int nd_place(mp_ctx *ctx, NdState *s) {
     return MP_OK;
 }
 
-// Builds the plan on the first direct solve after mp_fe_setup, and places it when
-// it is first the faster way.  *usable: the sparse factorization applies (K has the
-// mesh's pattern and is symmetric), is expected to be faster than the dense one
-// and has its memory; a device too full for it is asked again by the next call.
-int nd_prepare(mp_ctx *ctx, bool mixed, bool *usable) {
-    *usable = false;
+static int nd_plan_and_place(mp_ctx *ctx, bool mixed, bool *usable) {
     NdState *s = state_of(ctx);
     int rc;
     if (!s) {
@@ -1187,6 +1183,21 @@ int nd_prepare(mp_ctx *ctx, bool mixed, bool *usable) {
     }
     *usable = s->usable;
     return MP_OK;
+}
+
+// Builds the plan on the first direct solve after mp_fe_setup, and places it when
+// it is first the faster way.  *usable: the sparse factorization applies (K has the
+// mesh's pattern and is symmetric), is expected to be faster than the dense one
+// and has its memory.  Where the device or the host is too full for it, the dense
+// one takes the call and the next call asks again.
+int nd_prepare(mp_ctx *ctx, bool mixed, bool *usable) {
+    *usable = false;
+    try {
+        return nd_plan_and_place(ctx, mixed, usable);
+    } catch (const std::exception &) {
+        nd_free(ctx);
+        return MP_OK;
+    }
 }
 
 static int nd_launch_solve(mp_ctx *ctx, NdState *s, bool back, const double *b, double *y, bool add) {

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <exception>
 #include <future>
 #include <limits>
 #include <numeric>
@@ -164,10 +165,15 @@ struct Dissection {
         s.shrink_to_fit();
         if (depth < 3 && a.size() + b.size() > 4000) {
             std::vector<Part> pa;
-            auto f = std::async(std::launch::async, [&] { run(std::move(a), depth + 1, pa); });
+            std::future<void> f;
+            try {
+                f = std::async(std::launch::async, [&] { run(std::move(a), depth + 1, pa); });
+            } catch (const std::exception &) {  // no thread can be had: one side after the other
+            }
+            if (!f.valid()) run(std::move(a), depth + 1, pa);
             std::vector<Part> pb;
             run(std::move(b), depth + 1, pb);
-            f.get();
+            if (f.valid()) f.get();
             for (auto &p : pa) out.push_back(std::move(p));
             for (auto &p : pb) out.push_back(std::move(p));
         } else {
