@@ -709,7 +709,8 @@ int mp_adjoint_forward(mp_ctx *ctx, const double *phi, double v_drift, int mode,
     }
     if (ctx->counters_host[C_FLAGS] & FLAG_WALK_LIMIT) {
         unsigned long long keep = ctx->counters_host[C_FLAGS] & ~FLAG_WALK_LIMIT;
-        MP_CUDA(ctx, cudaMemcpy(ctx->counters + C_FLAGS, &keep, sizeof(keep), cudaMemcpyHostToDevice));
+        MP_CUDA(ctx, upload(ctx, ctx->counters + C_FLAGS, &keep, sizeof(keep)));
+        MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         return fail(ctx, MP_ERR_WALK_LIMIT, "adjoint forward: a tet walk exceeded the hop limit");
     }
     return MP_OK;

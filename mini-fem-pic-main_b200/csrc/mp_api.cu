@@ -701,7 +701,7 @@ int mp_fe_setup(mp_ctx *ctx, const mp_fe_desc *fe) {
     double **vp[] = {&ctx->d, &ctx->F0, &ctx->F1, &ctx->G, &ctx->y, &ctx->fvec, &ctx->FP, &ctx->work};
     for (double **p : vp) {
         MP_CUDA(ctx, cudaMalloc(p, vec));
-        MP_CUDA(ctx, cudaMemset(*p, 0, vec));
+        MP_CUDA(ctx, cudaMemsetAsync(*p, 0, vec, ctx->stream));
     }
     ctx->K = ctx->J = nullptr;  // J: allocated when an FP64 dense J is first built
     ctx->j32_current = ctx->j_current = ctx->j_dense = ctx->fp_is_j = false;
@@ -730,17 +730,17 @@ int mp_fe_setup(mp_ctx *ctx, const mp_fe_desc *fe) {
     if (fe->K_rows || fe->K_dense) {
         if (!fe->F0) return fail(ctx, MP_ERR_ARG, "K given without F0");
         if (dense) {
-            MP_CUDA(ctx, cudaMemset(ctx->K, 0, sizeof(double) * (size_t)ld * neq));
+            MP_CUDA(ctx, cudaMemsetAsync(ctx->K, 0, sizeof(double) * (size_t)ld * neq, st));
             for (int i = 0; i < neq; i++) {
                 const double *row = fe->K_rows ? fe->K_rows[i] : fe->K_dense + (size_t)i * neq;
-                MP_CUDA(ctx, cudaMemcpy(ctx->K + (size_t)i * ld, row, sizeof(double) * neq, cudaMemcpyHostToDevice));
+                MP_CUDA(ctx, upload(ctx, ctx->K + (size_t)i * ld, row, sizeof(double) * neq));
             }
             rc = fe_sparse_from_dense(ctx);
         } else {
             rc = fe_sparse_from_host(ctx, fe->K_rows, fe->K_dense);
         }
         if (rc) return rc;
-        MP_CUDA(ctx, cudaMemcpy(ctx->F0, fe->F0, sizeof(double) * neq, cudaMemcpyHostToDevice));
+        MP_CUDA(ctx, upload(ctx, ctx->F0, fe->F0, sizeof(double) * neq));
     } else {
         rc = dense ? fe_assemble(ctx) : fe_assemble_sparse(ctx);
         if (rc) return rc;
@@ -821,8 +821,8 @@ int mp_fe_upload(mp_ctx *ctx, int which, const double *values) {
                 rec[e].ef[d] = ef[3 * (size_t)e + d];
                 rec32[e].ef[d] = (float)ef[3 * (size_t)e + d];
             }
-        MP_CUDA(ctx, cudaMemcpy(ctx->tets, rec.data(), sizeof(TetRec) * ctx->n_tets, cudaMemcpyHostToDevice));
-        MP_CUDA(ctx, cudaMemcpy(ctx->tets32, rec32.data(), sizeof(TetRec32) * ctx->n_tets, cudaMemcpyHostToDevice));
+        MP_CUDA(ctx, upload(ctx, ctx->tets, rec.data(), sizeof(TetRec) * ctx->n_tets));
+        MP_CUDA(ctx, upload(ctx, ctx->tets32, rec32.data(), sizeof(TetRec32) * ctx->n_tets));
     }
     MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return MP_OK;

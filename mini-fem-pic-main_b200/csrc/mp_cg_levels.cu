@@ -1198,7 +1198,7 @@ static int make_plan(mp_ctx *ctx, Plan *p, const std::vector<long long> &rowp, c
     if (!device_room((void **)&p->blob, off)) return MP_OK;  // unusable, no error
     unsigned char *base = static_cast<unsigned char *>(p->blob);
 #define X(v) \
-    if (!v.empty()) MP_CUDA(ctx, cudaMemcpy(base + o_##v, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
+    if (!v.empty()) MP_CUDA(ctx, upload(ctx, base + o_##v, v.data(), v.size() * sizeof(v[0])));
     CG_ARRAYS(X)
 #undef X
 #undef CG_ARRAYS
@@ -1230,6 +1230,7 @@ static int make_plan(mp_ctx *ctx, Plan *p, const std::vector<long long> &rowp, c
     a.sums = at(o_sums);
     a.flag = reinterpret_cast<unsigned *>(base + o_flag);
     MP_CUDA(ctx, cudaMemsetAsync(a.share, 0, 16 * (size_t)a.shares, ctx->stream));  // the odd functions' last places stay zero
+    MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     p->usable = true;
     return MP_OK;
 }

@@ -346,7 +346,7 @@ static int gs_plan(mp_ctx *ctx, bool *usable) {
             return MP_OK;
         }
         char *base = static_cast<char *>(s->blob);
-        for (int k = 0; k < 8; k++) MP_CUDA(ctx, cudaMemcpy(base + off[k], src[k], bytes[k], cudaMemcpyHostToDevice));
+        for (int k = 0; k < 8; k++) MP_CUDA(ctx, upload(ctx, base + off[k], src[k], bytes[k]));
         MP_CUDA(ctx, cudaHostAlloc(&s->out_host, sizeof(double) * 4, 0));
         const int most = (int)sizeof(double) * 1024 * GS_MAX_CLUSTER;
         MP_CUDA(ctx, cudaFuncSetAttribute(k_gs_cluster<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
@@ -359,6 +359,7 @@ static int gs_plan(mp_ctx *ctx, bool *usable) {
         s->a.due = reinterpret_cast<const int *>(base + off[5]);
         s->a.near = reinterpret_cast<const int *>(base + off[6]);
         s->a.to = reinterpret_cast<const unsigned char *>(base + off[7]);
+        MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         s->a.n = n;
         s->a.levels = levels;
         s->a.distance = distance;

@@ -145,8 +145,9 @@ extern "C" int mp_inject_device(mp_ctx *ctx, mp_injector *inj, double plasma_den
         MP_CUDA(ctx, cudaMalloc(&s->face_cell, sizeof(int) * (nf + 1)));
         MP_CUDA(ctx, cudaMalloc(&s->prefix, sizeof(int) * (nf + 1)));
         MP_CUDA(ctx, cudaMallocHost(&s->prefix_host, sizeof(int) * (nf + 1)));
-        MP_CUDA(ctx, cudaMemcpy(s->faces, fh.data(), sizeof(double) * fh.size(), cudaMemcpyHostToDevice));
-        MP_CUDA(ctx, cudaMemcpy(s->face_cell, inj->cell.data(), sizeof(int) * nf, cudaMemcpyHostToDevice));
+        MP_CUDA(ctx, upload(ctx, s->faces, fh.data(), sizeof(double) * fh.size()));
+        MP_CUDA(ctx, upload(ctx, s->face_cell, inj->cell.data(), sizeof(int) * nf));
+        MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         s->inj = inj;
         s->n_faces = nf;
     }

@@ -252,6 +252,12 @@ int cuda_fail(mp_ctx *ctx, cudaError_t e, const char *what);
 // Kernels' host launchers (push / field / solver translation units).
 int ensure_dstage(mp_ctx *ctx, size_t bytes);
 bool device_room(void **p, size_t bytes);
+// Host to device in the order of the context's stream, whose kernels read it: the stream is
+// a non-blocking one, which a plain cudaMemcpy's last part (it may return before that has
+// arrived) is not ordered with.  The caller waits for the stream before a pinned source goes.
+inline cudaError_t upload(mp_ctx *ctx, void *dst, const void *src, size_t bytes) {
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
+}
 int launch_push(mp_ctx *ctx, double q_over_m, double dt);
 int launch_normalise(mp_ctx *ctx, double spwt);
 int launch_append(mp_ctx *ctx, long long n, const double *pos_soa, const double *vel_soa, const int *cell,

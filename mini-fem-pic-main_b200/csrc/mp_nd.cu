@@ -1131,7 +1131,7 @@ static int nd_place(mp_ctx *ctx, NdState *s) {
                        {(void **)&s->ctl, sizeof(unsigned) * 8}},
                       device_room, cudaFree))
         return MP_OK;
-    MP_CUDA(ctx, cudaMemcpy(s->blob, host.data(), host.size(), cudaMemcpyHostToDevice));
+    MP_CUDA(ctx, upload(ctx, s->blob, host.data(), host.size()));
 #define X(a) s->a = reinterpret_cast<decltype(s->a)>(static_cast<unsigned char *>(s->blob) + o_##a);
     ND_ARRAYS(X)
 #undef X
@@ -1145,6 +1145,7 @@ static int nd_place(mp_ctx *ctx, NdState *s) {
                                       (int)sizeof(SolveSmem)));
     MP_CUDA(ctx, cudaFuncSetAttribute(k_nd_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)sizeof(SolveSmem)));
+    MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     p.task.clear();
     p.task.shrink_to_fit();
     p.item.clear();

@@ -510,10 +510,11 @@ int sparse_setup(mp_ctx *ctx, const std::vector<int> &LM, const std::vector<int>
     MP_CUDA(ctx, cudaMalloc(&ctx->sp_ptr, sizeof(long long) * (slices + 1)));
     MP_CUDA(ctx, cudaMalloc(&ctx->sp_col, sizeof(int) * std::max(1ll, slots)));
     MP_CUDA(ctx, cudaMalloc(&ctx->sp_val, sizeof(double) * std::max(1ll, slots)));
-    MP_CUDA(ctx, cudaMemcpy(ctx->sp_len, len.data(), sizeof(int) * neq, cudaMemcpyHostToDevice));
-    MP_CUDA(ctx, cudaMemcpy(ctx->sp_ptr, ptr.data(), sizeof(long long) * (slices + 1), cudaMemcpyHostToDevice));
-    if (slots) MP_CUDA(ctx, cudaMemcpy(ctx->sp_col, col.data(), sizeof(int) * slots, cudaMemcpyHostToDevice));
-    MP_CUDA(ctx, cudaMemset(ctx->sp_val, 0, sizeof(double) * std::max(1ll, slots)));
+    MP_CUDA(ctx, upload(ctx, ctx->sp_len, len.data(), sizeof(int) * neq));
+    MP_CUDA(ctx, upload(ctx, ctx->sp_ptr, ptr.data(), sizeof(long long) * (slices + 1)));
+    if (slots) MP_CUDA(ctx, upload(ctx, ctx->sp_col, col.data(), sizeof(int) * slots));
+    MP_CUDA(ctx, cudaMemsetAsync(ctx->sp_val, 0, sizeof(double) * std::max(1ll, slots), ctx->stream));
+    MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     ctx->sp_nnz = nnz;
     ctx->sp_slots = slots;
     ctx->csr_ptr.clear();
@@ -624,7 +625,8 @@ int fe_sparse_from_host(mp_ctx *ctx, const double *const *rows, const double *de
         for (int k = 0; k < len[P]; k++) val[base + 32ll * k] = row[col[base + 32ll * k]];
     }
     if (ctx->sp_slots)
-        MP_CUDA(ctx, cudaMemcpy(ctx->sp_val, val.data(), sizeof(double) * ctx->sp_slots, cudaMemcpyHostToDevice));
+        MP_CUDA(ctx, upload(ctx, ctx->sp_val, val.data(), sizeof(double) * ctx->sp_slots));
+    MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return MP_OK;
 }
 
