@@ -273,12 +273,12 @@ int launch_update_ef(mp_ctx *ctx);
 // direct solve, deciding on the device whether its solution is taken; the update
 // of d and uh, unless *stop, with the step's scalars on their way to the host.
 struct NewtonState {
-    double l2, rn, bn;            // ||y|| / neq, ||G - J y||, ||G||
+    double l2, rn, of;            // ||y|| / neq, ||G - J y||, what the check related that to
     bool taken;
     unsigned long long flags;
 };
 int newton_terms(mp_ctx *ctx, const double *den, bool clear_y, unsigned *clear, int clear_words);
-int newton_check(mp_ctx *ctx, double rtol, unsigned long long bad_flags);
+int newton_check(mp_ctx *ctx, double rtol, bool terms, unsigned long long bad_flags);
 const unsigned *newton_go(mp_ctx *ctx);
 int newton_update(mp_ctx *ctx, const unsigned *stop);
 void newton_read(mp_ctx *ctx, NewtonState *s);

@@ -17,7 +17,7 @@ constexpr int STEP_THREADS = 128;
 constexpr int CHECK_TEAM = 16;  // lanes that share one row
 
 // Words of ctx->scal (8 doubles) that a step uses.
-enum { S_Y2 = 0, S_R2 = 1, S_B2 = 2, S_GO = 5, S_FLAGS = 6, S_TICKET = 7 };
+enum { S_Y2 = 0, S_R2 = 1, S_OF2 = 2, S_GO = 5, S_FLAGS = 6, S_TICKET = 7 };
 
 // value of lane k of the team, k < TEAM
 template <int TEAM>
@@ -118,55 +118,65 @@ struct CheckArgs {
     unsigned long long bad;            // flag bits that refuse the solution
     int neq;
     double rtol;
+    bool terms;                        // relative to r's terms, not to b
 };
 
-// r = b - (K y - FP .* y), its norm and b's; the last block decides whether the
-// solution is taken (S_GO = 0): ||r|| <= rtol ||b|| and none of the bad flags.
+// r = b - (K y - FP .* y), its norm and b's, or that of the terms r is the sum of, |b| + |K| |y|
+// + |FP| |y|; the last block decides whether the solution is taken (S_GO = 0): the first norm
+// <= rtol times the second and none of the bad flags.
 template <int TEAM>
 __global__ void __launch_bounds__(STEP_THREADS) k_newton_check(CheckArgs a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & (TEAM - 1);
     const int P = i / TEAM;
-    double s = 0.0, rr = 0.0, bb = 0.0;
+    double s = 0.0, t = 0.0, rr = 0.0, oo = 0.0;
     if (P < a.neq) {
         const long long row = a.sp_ptr[P >> 5] + (P & 31);
         const int len = a.sp_len[P];
-        for (int k = lane; k < len; k += TEAM) s = fma(a.sp_val[row + 32ll * k], a.y[a.sp_col[row + 32ll * k]], s);
+        for (int k = lane; k < len; k += TEAM) {
+            const double v = a.sp_val[row + 32ll * k], x = a.y[a.sp_col[row + 32ll * k]];
+            s = fma(v, x, s);
+            t = fma(fabs(v), fabs(x), t);
+        }
     }
 #pragma unroll
-    for (int o = TEAM / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    for (int o = TEAM / 2; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        t += __shfl_xor_sync(0xffffffffu, t, o);
+    }
     if (P < a.neq && lane == 0) {
-        const double v = a.b[P] - (s - a.FP[P] * a.y[P]);
+        const double fy = a.FP[P] * a.y[P], v = a.b[P] - (s - fy);
         a.r[P] = v;
         rr = v * v;
-        bb = a.b[P] * a.b[P];
+        const double of = a.terms ? t + fabs(fy) + fabs(a.b[P]) : a.b[P];
+        oo = of * of;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         rr += __shfl_xor_sync(0xffffffffu, rr, o);
-        bb += __shfl_xor_sync(0xffffffffu, bb, o);
+        oo += __shfl_xor_sync(0xffffffffu, oo, o);
     }
     __shared__ double part[2][STEP_THREADS / 32];
     if ((threadIdx.x & 31) == 0) {
         part[0][threadIdx.x >> 5] = rr;
-        part[1][threadIdx.x >> 5] = bb;
+        part[1][threadIdx.x >> 5] = oo;
     }
     __syncthreads();
     if (threadIdx.x) return;
     for (int w = 1; w < STEP_THREADS / 32; w++) {
         rr += part[0][w];
-        bb += part[1][w];
+        oo += part[1][w];
     }
     atomicAdd(a.scal + S_R2, rr);
-    atomicAdd(a.scal + S_B2, bb);
+    atomicAdd(a.scal + S_OF2, oo);
     __threadfence();
     unsigned *ticket = reinterpret_cast<unsigned *>(a.scal + S_TICKET);
     if (atomicAdd(ticket, 1u) + 1 < gridDim.x) return;
     __threadfence();
     *ticket = 0;
-    const double r2 = __ldcg(a.scal + S_R2), b2 = __ldcg(a.scal + S_B2);
+    const double r2 = __ldcg(a.scal + S_R2), of2 = __ldcg(a.scal + S_OF2);
     const unsigned long long fl = *reinterpret_cast<const volatile unsigned long long *>(a.flags) & a.bad;
     *reinterpret_cast<unsigned long long *>(a.scal + S_FLAGS) = fl;
-    *reinterpret_cast<unsigned *>(a.scal + S_GO) = sqrt(r2) <= a.rtol * sqrt(b2) && !fl ? 0u : 1u;
+    *reinterpret_cast<unsigned *>(a.scal + S_GO) = sqrt(r2) <= a.rtol * sqrt(of2) && !fl ? 0u : 1u;
 }
 
 // d -= y with sum y^2, and uh = g + d (src/FESolver.cpp:341-349, 610-618), unless *stop
@@ -237,7 +247,7 @@ int newton_terms(mp_ctx *ctx, const double *den, bool clear_y, unsigned *clear, 
     return MP_OK;
 }
 
-int newton_check(mp_ctx *ctx, double rtol, unsigned long long bad_flags) {
+int newton_check(mp_ctx *ctx, double rtol, bool terms, unsigned long long bad_flags) {
     CheckArgs a;
     a.sp_len = ctx->sp_len;
     a.sp_col = ctx->sp_col;
@@ -252,6 +262,7 @@ int newton_check(mp_ctx *ctx, double rtol, unsigned long long bad_flags) {
     a.bad = bad_flags;
     a.neq = ctx->neq;
     a.rtol = rtol;
+    a.terms = terms;
     const unsigned blocks = (unsigned)(((long long)ctx->neq * CHECK_TEAM + STEP_THREADS - 1) / STEP_THREADS);
     k_newton_check<CHECK_TEAM><<<blocks, STEP_THREADS, 0, ctx->stream>>>(a), ++ctx->launches;
     MP_CUDA(ctx, cudaGetLastError());
@@ -273,7 +284,7 @@ int newton_update(mp_ctx *ctx, const unsigned *stop) {
 void newton_read(mp_ctx *ctx, NewtonState *s) {
     s->l2 = std::sqrt(ctx->scal_host[S_Y2]) / ctx->neq;
     s->rn = std::sqrt(ctx->scal_host[S_R2]);
-    s->bn = std::sqrt(ctx->scal_host[S_B2]);
+    s->of = std::sqrt(ctx->scal_host[S_OF2]);
     unsigned go;
     std::memcpy(&go, ctx->scal_host + S_GO, sizeof(go));
     s->taken = go == 0;

@@ -46,11 +46,12 @@ __global__ void k_axpy_f32(int n, const float *__restrict__ c, double *y) {
 }
 
 // r = b - J y and the norms ||r||, ||b||: from the sparse copy of K (about 15
-// nonzeros a row) when the context holds one, else from the dense K.
+// nonzeros a row) when the context holds one, else from the dense K.  sn, from the
+// sparse copy only: the norm of r's terms, |b| + |K| |y| + |FP| |y|.
 static int resid_norms(mp_ctx *ctx, const double *y, const double *b, double *r, float *r32, double *rn,
-                       double *bn) {
+                       double *bn, double *sn = nullptr) {
     long long ld = (ctx->neq + 31) & ~31ll;
-    MP_CUDA(ctx, cudaMemsetAsync(ctx->scal + 1, 0, 2 * sizeof(double), ctx->stream));
+    MP_CUDA(ctx, cudaMemsetAsync(ctx->scal + 1, 0, 3 * sizeof(double), ctx->stream));
     if (ctx->sp_val) {
         int rc = fe_resid_j_sparse(ctx, y, b, r, r32, ctx->scal + 1);
         if (rc) return rc;
@@ -61,11 +62,12 @@ static int resid_norms(mp_ctx *ctx, const double *y, const double *b, double *r,
             ++ctx->launches;
     }
     MP_CUDA(ctx, cudaGetLastError());
-    MP_CUDA(ctx, cudaMemcpyAsync(ctx->scal_host + 1, ctx->scal + 1, 2 * sizeof(double), cudaMemcpyDeviceToHost,
+    MP_CUDA(ctx, cudaMemcpyAsync(ctx->scal_host + 1, ctx->scal + 1, 3 * sizeof(double), cudaMemcpyDeviceToHost,
                                  ctx->stream));
     MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     *rn = std::sqrt(ctx->scal_host[1]);
     *bn = std::sqrt(ctx->scal_host[2]);
+    if (sn) *sn = std::sqrt(ctx->scal_host[3]);
     return MP_OK;
 }
 
@@ -154,27 +156,37 @@ constexpr double GS_TOL = 1e-4;  // solveLinear's ||b - A x|| / neq, src/FESolve
 
 static int solve_dense(mp_ctx *ctx, int form, mp_newton_stats *st);
 
-// A residual above this share of ||G|| (an indefinite J can meet a bad pivot
-// order) sends the sparse factorization's solve to the dense one.
-constexpr double SPARSE_RTOL = 1e-9;
+// A solve by the sparse factor, which does not pivot, is as good as a stable one when
+// its residual is that of rounding, relative to the terms it is the sum of: ||r|| <=
+// this ||s||, s = |G| + |K| |y| + |FP| |y|.  ||r|| / ||s|| is 1.0e-16 to 1.9e-16 on boxes and
+// Delaunay meshes of 144 to 32,244 unknowns; small pivots of an indefinite J raised it
+// to 2e-10 (y off by 2e-9 at a condition of 100), and a refinement pass took it to 6e-17.
+constexpr double SOUND = 4 * 0x1p-53;
 
-// The direct solve by the sparse factorization; *done is false when the dense
-// one has to take it over (a zero or non-finite pivot, a poor residual).
-// enqueued: nd_factor_solve and newton_check have run, rn and bn hold their norms.
-static int solve_nd(mp_ctx *ctx, int form, mp_newton_stats *st, bool *done, bool enqueued, double rn, double bn) {
+// The direct solve by the sparse factorization, refined until its residual is that
+// of rounding (FP64 form) or REFINE_RTOL ||G|| (mixed form) or stalls; *done is
+// false when the dense one has to take it over (a zero or non-finite pivot, a residual
+// that refinement does not bring down).  enqueued: nd_factor_solve and newton_check
+// have run, with the norms rn and of.
+static int solve_nd(mp_ctx *ctx, int form, mp_newton_stats *st, bool *done, bool enqueued, double rn, double of) {
     *done = false;
+    const bool fp64 = form == MP_FORM_FP64;
+    const double rtol = fp64 ? SOUND : REFINE_RTOL;
+    double bn = 0, sn = 0;
     int rc;
     if (!enqueued) {
         cudaEventRecord(ctx->t1.a, ctx->stream);
         if ((rc = nd_factor_solve(ctx, ctx->G, ctx->y))) return rc;
         cudaEventRecord(ctx->t1.b, ctx->stream);
-        if ((rc = resid_norms(ctx, ctx->y, ctx->G, ctx->work, nullptr, &rn, &bn))) return rc;
     }
     double prev = 1e300;
     int it = 1;
     for (; it < 60; it++) {
-        if (it > 1 && (rc = resid_norms(ctx, ctx->y, ctx->G, ctx->work, nullptr, &rn, &bn))) return rc;
-        if (form == MP_FORM_FP64 || !(rn > REFINE_RTOL * bn) || !(rn <= SPARSE_RTOL * bn) || rn > 0.7 * prev) break;
+        if (it > 1 || !enqueued) {
+            if ((rc = resid_norms(ctx, ctx->y, ctx->G, ctx->work, nullptr, &rn, &bn, &sn))) return rc;
+            of = fp64 ? sn : bn;
+        }
+        if (rn <= rtol * of || !(rn <= 0.7 * prev)) break;
         prev = rn;
         if ((rc = nd_solve_add(ctx, ctx->work, ctx->y))) return rc;
     }
@@ -182,7 +194,7 @@ static int solve_nd(mp_ctx *ctx, int form, mp_newton_stats *st, bool *done, bool
     if ((rc = check_flags(ctx, FLAG_SINGULAR | FLAG_LOOKBACK_TIMEOUT, &bad))) return rc;
     if (bad & FLAG_LOOKBACK_TIMEOUT)
         return fail(ctx, MP_ERR_TIMEOUT, "a bounded wait in the factorization or the triangular solves gave up");
-    if (bad || !(rn <= SPARSE_RTOL * bn)) return MP_OK;
+    if (bad || !(rn <= rtol * of || rn <= SOUND * sn)) return MP_OK;
     if (st) {
         st->linear_iterations = it;
         st->linear_residual = rn / ctx->neq;
@@ -216,8 +228,8 @@ int fe_step_lean(mp_ctx *ctx, const double *den, int method, int form, bool firs
         cudaEventRecord(ctx->t1.a, ctx->stream);
         if ((rc = nd_factor_solve(ctx, ctx->G, ctx->y, true))) return rc;
         cudaEventRecord(ctx->t1.b, ctx->stream);
-        if ((rc = newton_check(ctx, form == MP_FORM_FP64 ? SPARSE_RTOL : REFINE_RTOL,
-                               FLAG_SINGULAR | FLAG_LOOKBACK_TIMEOUT)))
+        const bool fp64 = form == MP_FORM_FP64;
+        if ((rc = newton_check(ctx, fp64 ? SOUND : REFINE_RTOL, fp64, FLAG_SINGULAR | FLAG_LOOKBACK_TIMEOUT)))
             return rc;
         stop = newton_go(ctx);
     }
@@ -248,7 +260,7 @@ int fe_step_lean(mp_ctx *ctx, const double *den, int method, int form, bool firs
         return MP_OK;
     }
     bool done = false;
-    if ((rc = solve_nd(ctx, form, st, &done, true, s.rn, s.bn))) return rc;
+    if ((rc = solve_nd(ctx, form, st, &done, true, s.rn, s.of))) return rc;
     if (!done) {
         if (form == MP_FORM_FP64) ctx->j_current = true;
         if ((rc = solve_dense(ctx, form, st))) return rc;

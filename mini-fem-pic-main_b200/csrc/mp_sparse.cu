@@ -632,18 +632,25 @@ int fe_sparse_from_host(mp_ctx *ctx, const double *const *rows, const double *de
 
 // r = b - (K y - FP .* y) from the sparse K (a refinement residual reads 12 B
 // per nonzero instead of the dense K's 8 neq^2 bytes); also emits r in FP32
-// and adds ||r||^2, ||b||^2 into sums[0], sums[1] (one atomic per warp).
+// and adds ||r||^2, ||b||^2 and ||s||^2, s = |b| + |K| |y| + |FP| |y|, into sums[0..2] (one
+// atomic each per warp).
 __global__ void k_resid_j_sparse(int neq, const int *__restrict__ len, const long long *__restrict__ ptr,
                                  const int *__restrict__ col, const double *__restrict__ val,
                                  const double *__restrict__ FP, const double *__restrict__ y,
                                  const double *__restrict__ b, double *r, float *r32, double *sums) {
     const int P = blockIdx.x * blockDim.x + threadIdx.x;
-    double rr = 0.0, bb = 0.0;
+    double rr = 0.0, bb = 0.0, tt = 0.0;
     if (P < neq) {
         const long long base = ptr[P >> 5] + (P & 31);
-        double sacc = 0.0;
-        for (int k = 0; k < len[P]; k++) sacc = fma(val[base + 32ll * k], y[col[base + 32ll * k]], sacc);
+        double sacc = 0.0, t = 0.0;
+        for (int k = 0; k < len[P]; k++) {
+            const double a = val[base + 32ll * k], x = y[col[base + 32ll * k]];
+            sacc = fma(a, x, sacc);
+            t = fma(fabs(a), fabs(x), t);
+        }
         const double v = b[P] - (sacc - FP[P] * y[P]);
+        t += fabs(FP[P] * y[P]) + fabs(b[P]);
+        tt = t * t;
         if (r) r[P] = v;
         if (r32) r32[P] = (float)v;
         rr = v * v;
@@ -653,10 +660,12 @@ __global__ void k_resid_j_sparse(int neq, const int *__restrict__ len, const lon
     for (int o = 16; o > 0; o >>= 1) {
         rr += __shfl_xor_sync(0xffffffffu, rr, o);
         bb += __shfl_xor_sync(0xffffffffu, bb, o);
+        tt += __shfl_xor_sync(0xffffffffu, tt, o);
     }
     if ((threadIdx.x & 31) == 0) {
         atomicAdd(&sums[0], rr);
         atomicAdd(&sums[1], bb);
+        atomicAdd(&sums[2], tt);
     }
 }
 
