@@ -469,7 +469,9 @@ int mp_adjoint_setup(mp_ctx *ctx, int32_t steps, int32_t checkpoint_every, doubl
                      int record_path);
 /* Adds n particles entering at first_step (0 = the initial population).
  * pos/vel packed [n][3]; injected != 0: vel is the thermal part v_th and the
- * drift and rewind are applied as above; injected == 0: vel is the velocity. */
+ * drift and rewind are applied as above; injected == 0: vel is the velocity.
+ * The arrays are host or device memory; device memory is read after the work
+ * enqueued so far in the default (legacy) stream, as by a plain cudaMemcpy. */
 int mp_adjoint_add_particles(mp_ctx *ctx, int32_t first_step, int injected, int64_t n, const double *pos,
                              const double *vel, const int32_t *cell);
 /* Runs the K steps: den_out [n_nodes] (nullable), stats (nullable).  Keeps the

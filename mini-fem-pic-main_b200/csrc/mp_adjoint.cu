@@ -48,6 +48,7 @@ namespace mp {
 
 constexpr int ADJ_MAX_SEGMENT = 32;  // checkpoint interval limit (per-thread cell array)
 constexpr int ADJ_THREADS = 256;
+constexpr int64_t ADJ_PIECE = 1 << 19;  // particles staged at a time, 56 B each
 
 // path codes of the recorded walk (cells >= 0 are the step's end cell)
 constexpr int PATH_EXIT_OTHER = -1, PATH_EXIT_WALL = -2, PATH_HOP_LIMIT = -3;
@@ -459,17 +460,17 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_tangent(AdjArgs a, const do
     if (threadIdx.x == 0 && t != 0) atomicAdd(&a.scal[2], t);
 }
 
-// Slots s0 + i <- particle order[i] of the packed arrays pos, vel [n][3].
+// Slot s0 + to[i] <- particle i of the packed arrays pos, vel [n][3].
 __global__ void k_adj_place(long long n, const double *__restrict__ pos, const double *__restrict__ vel,
-                            const int *__restrict__ cell, const int *__restrict__ order, int first, unsigned char inj,
+                            const int *__restrict__ cell, const int *__restrict__ to, int first, unsigned char inj,
                             long long s0, double *px, double *py, double *pz, double *vx, double *vy, double *vz,
                             int *cell0, int *firsts, unsigned char *injs) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const long long q = order[i], o = s0 + i;
-    px[o] = pos[3 * q]; py[o] = pos[3 * q + 1]; pz[o] = pos[3 * q + 2];
-    vx[o] = vel[3 * q]; vy[o] = vel[3 * q + 1]; vz[o] = vel[3 * q + 2];
-    cell0[o] = cell[q];
+    const long long o = s0 + to[i];
+    px[o] = pos[3 * i]; py[o] = pos[3 * i + 1]; pz[o] = pos[3 * i + 2];
+    vx[o] = vel[3 * i]; vy[o] = vel[3 * i + 1]; vz[o] = vel[3 * i + 2];
+    cell0[o] = cell[i];
     firsts[o] = first;
     injs[o] = inj;
 }
@@ -632,29 +633,37 @@ int mp_adjoint_add_particles(mp_ctx *ctx, int32_t first_step, int injected, int6
     if (n == 0) return MP_OK;
     if (n > (1ll << 31) - 1) return fail(ctx, MP_ERR_ARG, "more than 2^31 - 1 adjoint particles in one call");
     // pos, vel and cell may be host or device memory; the slots' order by cell is made on the host
-    std::vector<int> c(n), order(n), at(ctx->n_tets + 1, 0);
+    std::vector<int> c(n), to(n), at(ctx->n_tets + 1, 0);
     MP_CUDA(ctx, cudaMemcpy(c.data(), cell, sizeof(int) * n, cudaMemcpyDefault));
     for (int64_t i = 0; i < n; i++) {
         if (c[i] < 0 || c[i] >= ctx->n_tets) return fail(ctx, MP_ERR_ARG, "adjoint particle cell out of range");
         at[c[i] + 1]++;
     }
     for (int t = 0; t < ctx->n_tets; t++) at[t + 1] += at[t];
-    for (int64_t i = 0; i < n; i++) order[at[c[i]]++] = (int)i;
+    for (int64_t i = 0; i < n; i++) to[i] = at[c[i]]++;
     int rc = grow_slots(ctx, s, s->n + n);
     if (rc) return rc;
-    if ((rc = ensure_dstage(ctx, (6 * sizeof(double) + 2 * sizeof(int)) * n))) return rc;
-    double *p3 = (double *)ctx->dstage, *v3 = p3 + 3 * n;
-    int *dc = (int *)(v3 + 3 * n), *dord = dc + n;
-    MP_CUDA(ctx, cudaMemcpyAsync(p3, pos, sizeof(double) * 3 * n, cudaMemcpyDefault, ctx->stream));
-    MP_CUDA(ctx, cudaMemcpyAsync(v3, vel, sizeof(double) * 3 * n, cudaMemcpyDefault, ctx->stream));
-    MP_CUDA(ctx, cudaMemcpyAsync(dc, c.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
-    MP_CUDA(ctx, cudaMemcpyAsync(dord, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
-    k_adj_place<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(
-        n, p3, v3, dc, dord, first_step, injected ? 1 : 0, s->n, s->px, s->py, s->pz, s->vx, s->vy, s->vz, s->cell0,
-        s->first, s->inj),
-        ++ctx->launches;
-    MP_CUDA(ctx, cudaGetLastError());
+    // Staged in pieces, so that the context keeps little memory for it, and all in the legacy
+    // stream: device memory is then read after the caller's work there, as by a plain cudaMemcpy.
+    const int64_t most = std::min(n, ADJ_PIECE);
+    if ((rc = ensure_dstage(ctx, (6 * sizeof(double) + 2 * sizeof(int)) * most))) return rc;
+    double *p3 = (double *)ctx->dstage, *v3 = p3 + 3 * most;
+    int *dc = (int *)(v3 + 3 * most), *dto = dc + most;
+    const cudaStream_t st = cudaStreamLegacy;
     MP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    for (int64_t q = 0; q < n; q += most) {
+        const int64_t m = std::min(most, n - q);
+        MP_CUDA(ctx, cudaMemcpyAsync(p3, pos + 3 * q, sizeof(double) * 3 * m, cudaMemcpyDefault, st));
+        MP_CUDA(ctx, cudaMemcpyAsync(v3, vel + 3 * q, sizeof(double) * 3 * m, cudaMemcpyDefault, st));
+        MP_CUDA(ctx, cudaMemcpyAsync(dc, c.data() + q, sizeof(int) * m, cudaMemcpyHostToDevice, st));
+        MP_CUDA(ctx, cudaMemcpyAsync(dto, to.data() + q, sizeof(int) * m, cudaMemcpyHostToDevice, st));
+        k_adj_place<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(m, p3, v3, dc, dto, first_step, injected ? 1 : 0, s->n,
+                                                                 s->px, s->py, s->pz, s->vx, s->vy, s->vz, s->cell0,
+                                                                 s->first, s->inj),
+            ++ctx->launches;
+        MP_CUDA(ctx, cudaGetLastError());
+    }
+    MP_CUDA(ctx, cudaStreamSynchronize(st));
     s->n += n;
     s->tape = false;
     s->path_valid = false;
