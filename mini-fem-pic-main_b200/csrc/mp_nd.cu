@@ -31,6 +31,7 @@
 #include "mp_alloc.h"
 #include "mp_internal.h"
 #include "mp_nd.h"
+#include "mp_recip.cuh"
 
 namespace mp {
 
@@ -364,17 +365,6 @@ __device__ __forceinline__ double sum_quad(double s) {
     return s;
 }
 
-// 1/d to a unit in the last place or so: the hardware approximation (2^-20 or
-// better) and one step of the third-order Householder iteration, for |d| in
-// [1e-290, 1e290] (a pivot outside is reported and the factor not used).  A
-// division's latency would be on the chain of pivots.
-__device__ __forceinline__ double reciprocal(double d) {
-    double x;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
-    const double e = fma(-d, x, 1.0);
-    return fma(x, fma(e, e, e), x);
-}
-
 // L D L^T of the 8 x 8 diagonal block s of sm.c in one warp, and the inverse of
 // its L: lane 4r + q holds columns q and q + 4 of row r, of the whole symmetric
 // block, so a pivot row is at hand in its own lanes' registers.  Two pivots a
@@ -393,6 +383,7 @@ __device__ __forceinline__ void factor8(Smem &sm, int s, int lane, unsigned long
         m[i] = c == r ? 1.0 : 0.0;
     }
     double pr = 1.0, gr = 0.0, cr = 1.0;  // the 2 x 2 block of this row's pair
+    bool sound = true;
 #pragma unroll
     for (int k = 0; k < 8; k += 2) {
         const int i = k >> 2, q0 = k & 3;
@@ -407,7 +398,9 @@ __device__ __forceinline__ void factor8(Smem &sm, int s, int lane, unsigned long
         if (k == 6) break;  // the last rows are done
         const double u = __shfl_sync(FULL, a[i], (lane & ~3) | q0);
         const double v = __shfl_sync(FULL, a[i], (lane & ~3) | (q0 + 1));
-        double rd = reciprocal(fma(p, c, -(g * g)));
+        const double det = fma(p, c, -(g * g));
+        sound &= invertible(det);
+        double rd = reciprocal(det);
         if (r <= k + 1) rd = 0.0;
         const double w0 = fma(g, v, -(c * u)) * rd, w1 = fma(g, u, -(p * v)) * rd;
 #pragma unroll
@@ -433,8 +426,8 @@ __device__ __forceinline__ void factor8(Smem &sm, int s, int lane, unsigned long
             m[1] = fma(-l, m1, m[1]);
         }
     }
-    // a pivot that the reciprocals could not take makes itself or a later one fail this
-    if (!(fabs(dr) > 1e-290) || !(fabs(dr) < 1e290)) atomicOr(flags, FLAG_SINGULAR);
+    // pr is the pivot of the pair's first row
+    if (!sound || !invertible(dr)) atomicOr(flags, FLAG_SINGULAR);
     if (q > r) m[0] = 0.0;
     if (q + 4 > r) m[1] = 0.0;
     *reinterpret_cast<double2 *>(sm.inv + s * 512 + s * 64 + 2 * lane) = make_double2(m[0], m[1]);
