@@ -155,7 +155,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_gs_cluster(GsArgs a) {
         const int steps = a.levels + a.distance * (S - 1);
         int turn = 0;                                  // step modulo distance
         unsigned bytes = near && t == 0 ? incoming(0, 0, S) : 0;
-        for (int w = 0; w < steps; w++, step++) {
+        int w = 0;
+        for (; w < steps && ok; w++, step++) {
             const unsigned bar = sm_addr(come + (step & 1));
             if (near && t == 0)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_gs_cluster(GsArgs a) {
             turn = turn + 1 == a.distance ? 0 : turn + 1;
             if (near && t == 0 && w + 1 < steps) bytes = incoming(w + 1, turn, S);
             __syncthreads();
-            for (unsigned i = 0; near && ok; i++) {
+            for (unsigned i = 0; near; i++) {
                 unsigned got;
                 asm volatile(
                     "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
@@ -179,9 +180,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_gs_cluster(GsArgs a) {
                     : "r"(bar), "r"((step >> 1) & 1)
                     : "memory");
                 if (got) break;
-                if (i > GS_SPIN_LIMIT) ok = false;     // the sweeps then run out without waiting, and the host is told
+                if (i > GS_SPIN_LIMIT) {               // a warp's lanes poll as one, and give up as one
+                    ok = false;
+                    break;
+                }
             }
         }
+        // After a wait that gave up: no arming, sending or waiting any more, so that a phase that
+        // never ends gets no second arrival and the other CTAs' waits give up too; the host is
+        // told.  (Within the noise: 432.3 us against 433.8 for 1,859 unknowns, 126 sweeps.)
+        for (; w < steps; w++) __syncthreads();
         done += S;
         if ((done - 1) % 25) break;                    // the sweep limit came before the next check
         double r = 0.0;
