@@ -442,10 +442,12 @@ static int grid_for(mp_ctx *ctx, const void *kernel, int threads, size_t smem) {
 
 // CTAs of a push: one wave of resident ones, or 3 to 8 waves of at least 4,096
 // particles a CTA.  A CTA's block of particles takes its time by their hops and
-// the mesh's band they lie in, and one wave ends with its slowest CTA: 48M ions
-// FP64 1.97 -> 1.51 ms, mixed 1.24 -> 1.00, 16M 665 -> 551 and 420 -> 375 us.  Two
-// waves, or smaller blocks, cost the L1's reuse more than they balance (mixed, 4M
-// ions: 97 us in one wave, 113 in two; FP64, 2M: 77, 80 and in four 87).
+// the mesh's band they lie in, and one wave ends with its slowest CTA.  On the 32^3
+// box minus the sphere, sorted every 10 steps, one wave -> by this rule: 39.2M ions
+// FP64 1,718 -> 1,361 us, mixed 1,111 -> 899; 13.1M 582 -> 498 and 375 -> 335.  Fewer
+// ions: more waves, or smaller blocks, cost the L1's reuse more than they balance (1, 2
+// and 3 waves: 4.1M ions mixed 122, 127, 131 us, FP64 192, 188, 189; 1.8M on the 20^3
+// box mixed 53, 59, 62, FP64 80, 88, 90).
 static long long push_ctas(long long blocks, long long resident, long long n) {
     if (blocks < resident) return blocks;
     const long long waves = std::min(8ll, n / (4096 * resident));

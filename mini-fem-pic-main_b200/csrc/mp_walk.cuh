@@ -12,8 +12,9 @@ constexpr double ONE_SIXTH = 1.0 / 6.0;
 // 32 bytes of a tet's record in one load (32-byte aligned, read-only).  A warp's
 // lanes read up to 32 records, and a load costs the L1 a pass per record whatever
 // its width: with 16-byte and scalar loads the mixed push kept the L1 at 74 % of
-// its rate.  Push kernel, before -> with these: mixed, 48M ions 1.23 -> 1.08 ms, 2M
-// 55 -> 51 us; FP64, 2M 85 -> 80 us.  (The mixed push's neighbours and nodes are
+// its rate.  Push kernel in one wave of CTAs, before -> with these: mixed, 39M ions on
+// the 32^3 box minus the sphere 1.23 -> 1.08 ms, 2M on the 20^3 box 55 -> 51 us; FP64, 2M
+// 85 -> 80 us.  (The mixed push's neighbours and nodes are
 // read when needed: loaded with the gradients they cost registers, 57 us at 2M.)
 __device__ __forceinline__ void load32(const double *p, double (&v)[4]) {
     asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
