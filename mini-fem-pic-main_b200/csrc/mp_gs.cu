@@ -305,6 +305,13 @@ static int gs_plan(mp_ctx *ctx, bool *usable) {
                 if (cluster > GS_MAX_CLUSTER) return MP_OK;
             }
         }
+        // 26 sweeps take 2 levels + 24 distance steps of 0.18 us in one CTA, 0.48 in a cluster of
+        // 512 threads a CTA, 0.68 of 1,024, and 40 us; dense sweeps 140 us and 0.43 us a row.  Numbers
+        // far from the coordinates' order make many levels and large distances: 144 rows numbered at
+        // random 294 us here, 232 dense; 567 rows 453 and 396, at random within slabs 640 and 395; but
+        // 1,859 rows at random 500 and 931.  By coordinate 60 to 214 us here, 163 to 3,970 dense.
+        const double step = cluster == 1 ? 0.18 : threads == 512 ? 0.48 : 0.68;
+        if (40 + (2.0 * levels + 24.0 * distance) * step > 140 + 0.43 * n) return MP_OK;
         const int P = (int)row.size();
         // who needs whose values
         std::vector<unsigned char> to(P, 0);
@@ -380,8 +387,8 @@ static int gs_plan(mp_ctx *ctx, bool *usable) {
 }
 
 // Plans the solve on its first use after mp_fe_setup.  *usable: every row fits
-// a thread and all rows one cluster of at most 8 CTAs, and K has the mesh's
-// pattern.  Where the device or the host is too full for the plan, the dense
+// a thread and all rows one cluster of at most 8 CTAs, K has the mesh's
+// pattern, and the rows' numbering makes this the faster way.  Where the device or the host is too full for the plan, the dense
 // sweeps take the call and the next call asks again.
 int gs_prepare(mp_ctx *ctx, bool *usable) {
     *usable = false;
