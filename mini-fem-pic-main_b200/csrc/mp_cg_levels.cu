@@ -886,10 +886,11 @@ static int make_plan(mp_ctx *ctx, Plan *p, const std::vector<long long> &rowp, c
             if (c <= limit) break;
             H *= 1.02;
         }
-        // A box one cell thick between planes of fixed nodes: its smooth errors die out across the
-        // box by themselves, and functions that do not vanish on the planes only cost.  0.05 x 1 x 1
-        // in units of the box, 245, 1,089 and 2,925 unknowns: 52, 83 and 88 iterations by levels in
-        // 0.33, 0.65 and 0.80 ms, 27, 57 and 88 by the diagonal in 0.21, 0.39 and 0.61.
+        // A thin box one cell thick between planes of fixed nodes: its smooth errors die out across
+        // the box by themselves, and functions that do not vanish on the planes only cost.  By levels
+        // and by the diagonal, unit boxes of 6^3 to 20^3 hexes made thinner: 0.01 to 0.03 of the
+        // extent 0.34 to 1.43 ms and 0.14 to 0.89, 0.05 (8^3 to 16^3) 0.36 to 0.87 and 0.33 to 0.78,
+        // 0.07 (8^3, 12^3) 0.34, 0.70 and 0.37, 0.56, but 0.1 (8^3, 10^3) 0.33, 0.43 and 0.42, 0.57.
         for (int d = 0; d < 3; d++) {
             double l = INFINITY, h = -INFINITY;
             for (int k = 0; k < ctx->n_nodes; k++)
@@ -898,7 +899,7 @@ static int make_plan(mp_ctx *ctx, Plan *p, const std::vector<long long> &rowp, c
                     h = std::max(h, npos[3 * (size_t)k + d]);
                 }
             const double edge = 1e-9 * ext[d];
-            if (cells[d] == 1 && l > lo[d] + edge && h < lo[d] + ext[d] - edge) return MP_OK;
+            if (cells[d] == 1 && 14 * ext[d] <= most && l > lo[d] + edge && h < lo[d] + ext[d] - edge) return MP_OK;
         }
         for (int k = 0; k < ctx->n_nodes; k++) {
             const int q = ID[k];
